@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "../../include/psb200.h"
+#include "psb_hanoi_words.cuh"
 #include "psb_internal.h"
 
 namespace psb {
@@ -133,7 +134,10 @@ __device__ __forceinline__ void engine_window(const LevelArgs& a, uint64_t windo
     if constexpr (T == kE_P10) level_window<PancakeK<10>, kTwoBit, kEThreads>(a, window, smem, sh);
     if constexpr (T == kE_P11) level_window<PancakeK<11>, kTwoBit, kEThreads>(a, window, smem, sh);
     if constexpr (T == kE_P12) level_window<PancakeK<12>, kTwoBit, kEThreads>(a, window, smem, sh);
-    if constexpr (T == kE_H) level_window<HanoiK, kTwoBit, kEThreads>(a, window, smem, sh);
+    if constexpr (T == kE_H) {
+        if (!hanoi_words_ok(a.pz)) level_window<HanoiK, kTwoBit, kEThreads>(a, window, smem, sh);
+        else if (!a.wflag_cur || a.wflag_cur[window]) hanoi_window<kTwoBit, kEThreads>(a, window, smem, sh);
+    }
 }
 
 template <int T>
