@@ -162,8 +162,8 @@ typedef struct {
                               PuzzleOptions::segmentBits, Common/DiskBasedBFS.h:11) */
     int32_t far_marks;     /* PSB_TWO_BIT top-down levels: where long-range marks go (PSB_FAR_*) */
     int32_t threads;       /* threads per block of the top-down two-bit and three-bit level kernels: 128, 256 or
-                              512 (0 = 128 for two-bit pancake and Hanoi searches of 2^32 states or more, else
-                              256); the other kernels use 256 */
+                              512 (0 = 128 for two-bit searches of Hanoi without symmetry, and of pancakes and
+                              symmetric Hanoi with 2^32 states or more; else 256); the other kernels use 256 */
     uint64_t* restored_counts; /* optional, counts_cap entries; 4-peg Hanoi with symmetry and PSB_TWO_BIT only:
                               the counts HanoiSearch reports (HanoiTowers/HanoiSearch.cpp:247-262), i.e. each
                               depth's canonical states weighted by their class size (PegsMult,

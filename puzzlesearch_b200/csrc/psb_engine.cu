@@ -135,8 +135,14 @@ __device__ __forceinline__ void engine_window(const LevelArgs& a, uint64_t windo
     if constexpr (T == kE_P11) level_window<PancakeK<11>, kTwoBit, kEThreads>(a, window, smem, sh);
     if constexpr (T == kE_P12) level_window<PancakeK<12>, kTwoBit, kEThreads>(a, window, smem, sh);
     if constexpr (T == kE_H) {
-        if (!hanoi_words_ok(a.pz)) level_window<HanoiK, kTwoBit, kEThreads>(a, window, smem, sh);
-        else if (!a.wflag_cur || a.wflag_cur[window]) hanoi_window<kTwoBit, kEThreads>(a, window, smem, sh);
+        if (!hanoi_words_ok(a.pz)) {
+            level_window<HanoiK, kTwoBit, kEThreads>(a, window, smem, sh);
+        } else if (!a.wflag_cur || a.wflag_cur[window]) {
+            HanoiCounts cnt;
+            hanoi_begin<kTwoBit, kEThreads>(a, smem, sh);
+            hanoi_window<kTwoBit, kEThreads>(a, window, smem, sh, cnt);
+            hanoi_end<kTwoBit>(a, cnt, sh);
+        }
     }
 }
 

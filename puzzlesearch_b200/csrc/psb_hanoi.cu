@@ -16,6 +16,8 @@ __global__ void __launch_bounds__(T, 1024 / T) hanoi_level_kernel(LevelArgs a, u
     extern __shared__ __align__(16) unsigned long long smem64[];
     __shared__ WindowShared sh;
     __shared__ uint32_t active[T / 32];
+    HanoiCounts cnt;
+    hanoi_begin<MODE, T>(a, smem64, sh);
     for (uint64_t g = blockIdx.x; g < n_windows; g += uint64_t(gridDim.x) * T) {
         const uint64_t mine = g + uint64_t(threadIdx.x) * gridDim.x;
         const bool on = mine < n_windows && (!a.wflag_cur || a.wflag_cur[mine]);
@@ -27,11 +29,12 @@ __global__ void __launch_bounds__(T, 1024 / T) hanoi_level_kernel(LevelArgs a, u
             while (m) {
                 const uint32_t j = __ffs(m) - 1;
                 m &= m - 1;
-                hanoi_window<MODE, T>(a, g + uint64_t(32 * i + j) * gridDim.x, smem64, sh);
+                hanoi_window<MODE, T>(a, g + uint64_t(32 * i + j) * gridDim.x, smem64, sh, cnt);
             }
         }
         __syncthreads();  // every thread has read active[]
     }
+    hanoi_end<MODE>(a, cnt, sh);
 }
 
 template <int MODE, int V = 0>

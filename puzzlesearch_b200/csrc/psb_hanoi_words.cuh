@@ -19,8 +19,9 @@
 // each state and was ALU-bound (76% of the ALU pipe, DRAM at 5%); a unit
 // takes about 250 here whatever number of its states is in the frontier.
 // Units holding frontier states are queued per warp and expanded 32 at a
-// time, so sparse chunks do not leave lanes idle.  What is left is the sweep
-// of the active windows and the shared-memory marks.
+// time, so sparse chunks do not leave lanes idle.  17 disks, two-bit, whole
+// search on B200: 444 -> 105 ms; a dense level of 15 disks 757 -> 191 us, the
+// ALU pipe at 52%, DRAM at 19%, a quarter of the stalls at window barriers.
 //
 // Marks of a unit are one 64-bit mask in shared memory (four for frontier
 // search, one per operator) in the unit's bit order, which is the order its
@@ -115,25 +116,69 @@ __host__ __device__ constexpr bool hanoi_words_ok(const PuzzleArgs& p) {
     return p.sym == 0 && p.disks >= 3 && p.disks <= 19;
 }
 
+// Chunks of 32 units that a warp sweeps at a time.
+__host__ __device__ constexpr int hanoi_group(int mode) { return mode == kFrontier ? 2 : 4; }
 // Shared memory of a window pass: the marks, then each warp's queue of units
-// (mask and unit number; at most 31 + 32 wait).
-constexpr uint32_t kHanoiQueue = 64;
+// (mask and unit number; at most 31 and a whole group wait).
+__host__ __device__ constexpr uint32_t hanoi_queue(int mode) { return 32u * (1 + hanoi_group(mode)); }
 __host__ __device__ constexpr size_t hanoi_queue_bytes(int mode) {
-    return kHanoiQueue * (8 * (mode == kFrontier ? 4 : 1) + 2);
+    return hanoi_queue(mode) * (8 * (mode == kFrontier ? 4 : 1) + 2);
 }
 __host__ __device__ constexpr size_t hanoi_smem_bytes(int mode, size_t window_states, int threads) {
     return mark_bytes(mode, window_states) + size_t(threads / 32) * hanoi_queue_bytes(mode);
 }
 
-// One window of a top-down level: level_window's contract, for searches with
-// hanoi_words_ok and a window that exists and is flagged (the caller looks).  The dynamic shared memory is level_window's (marks, then
-// each warp's list and scratch, which hold the warp's queue here).
+// A thread's share of the level's counters (LevelArgs::stats).
+struct HanoiCounts {
+    uint32_t found = 0, children = 0, remote = 0, next = 0, farmarks = 0;
+};
+
+// Clears the marks before a block's first window; hanoi_window leaves them
+// clear for the next.
+template <int MODE, int KTHREADS>
+__device__ __forceinline__ void hanoi_begin(const LevelArgs& a, unsigned long long* smem64, WindowShared& sh) {
+    const uint32_t mbytes = uint32_t(mark_bytes(MODE, size_t(1) << a.window_bits));
+    for (uint32_t i = threadIdx.x; i < mbytes / 16; i += KTHREADS)
+        reinterpret_cast<uint4*>(smem64)[i] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x == 0) {
+        sh.next_chunk = KTHREADS / 32;  // warp w's first group is group w
+        for (int i = 0; i < 8; ++i) sh.cnt[i] = 0;
+    }
+    __syncthreads();
+}
+
+// Adds the block's counters to the level's: one global atomic per block and counter.
+template <int MODE>
+__device__ __forceinline__ void hanoi_end(const LevelArgs& a, const HanoiCounts& c, WindowShared& sh) {
+    // signed: a unit's states are counted by the lane that sweeps it, its
+    // missing moves and remote children by the lane that expands it
+    const int32_t children = int32_t(c.children + (MODE != kFrontier ? 6 * c.found : 0));
+    const int32_t v[5] = {int32_t(c.found), children, children - int32_t(c.remote), int32_t(c.next),
+                          int32_t(c.farmarks)};
+    constexpr int kCounters = MODE == kTwoBit ? 5 : 3;
+#pragma unroll
+    for (int i = 0; i < kCounters; ++i) {
+        long long t = v[i];  // a block's windows can hold more than 2^32 children
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+        if ((threadIdx.x & 31) == 0 && t) atomicAdd(&sh.cnt[i < 3 ? i : i + 2], (unsigned long long)t);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 8; ++i)
+            if (sh.cnt[i]) atomicAdd(&a.stats[i], sh.cnt[i]);
+    }
+}
+
+// One window of a top-down level: level_window's contract between
+// hanoi_begin and hanoi_end, for searches with hanoi_words_ok and a window
+// that exists and is flagged (the caller looks).
 template <int MODE, int KTHREADS>
 __device__ __forceinline__ void hanoi_window(const LevelArgs& a, uint64_t window, unsigned long long* smem64,
-                                             WindowShared& sh) {
+                                             WindowShared& sh, HanoiCounts& cnt) {
     constexpr int kWarps = KTHREADS / 32;
     constexpr int kPlanes = MODE == kFrontier ? 4 : 1;
-    constexpr uint32_t kQueue = kHanoiQueue;
+    constexpr uint32_t kQueue = hanoi_queue(MODE);
     constexpr size_t kWarpBytes = hanoi_queue_bytes(MODE);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t W = 1u << a.window_bits;
@@ -147,14 +192,6 @@ __device__ __forceinline__ void hanoi_window(const LevelArgs& a, uint64_t window
     uint16_t* qunit = reinterpret_cast<uint16_t*>(qmask + kQueue * kPlanes);
     const uint32_t U0 = uint32_t(base >> 6);  // the window's first unit
     const uint32_t E = a.pz.disks == 19 ? 0x55555555u : 0x55555555u & ((1u << (2 * (a.pz.disks - 3))) - 1u);
-
-    for (uint32_t i = tid; i < mbytes / 16; i += KTHREADS) reinterpret_cast<uint4*>(smem64)[i] = make_uint4(0, 0, 0, 0);
-    if (tid == 0) {
-        sh.any = 0;
-        sh.next_chunk = kWarps;
-        for (int i = 0; i < 8; ++i) sh.cnt[i] = 0;
-    }
-    __syncthreads();
 
     uint32_t found = 0, children = 0, remote = 0, marked = 0, farmarks = 0;
     const uint32_t next_pat = 1u | (a.cur_code == 2 ? 2u : 0u);
@@ -230,38 +267,51 @@ __device__ __forceinline__ void hanoi_window(const LevelArgs& a, uint64_t window
             for (int p = 0; p < 4; ++p) mark_local(4 * u + p, out[p]);
         } else {
             mark_local(u, unit_moves<MODE, 0>(F) | unit_moves<MODE, 1>(F) | unit_moves<MODE, 2>(F));
-            children += 6 * __popcll(F);  // less the pairs with both pegs empty, below
+            // children: 6 per state, less the pairs with both pegs empty (below)
         }
-        // larger disks, one per peg pair
-        const uint32_t G[4] = {0, U >> 1, U, U ^ (U >> 1)};
-#pragma unroll
-        for (int x = 1; x < 4; ++x) {
-#pragma unroll
-            for (int v = 0; v < 2; ++v) {
-                uint64_t S = F & unit_free_mask<MODE>(x, v);
-                if (!S) continue;
-                const uint32_t e = (v ? G[x] : ~G[x]) & E;  // larger disks on the pair
-                const uint32_t k = e & (0u - e);            // the smallest of them
-                if (!k) {  // both pegs empty: no move
-                    if constexpr (MODE != kFrontier) children -= __popcll(S);
-                    continue;
-                }
-                uint32_t plane = 0;
-                if constexpr (MODE == kFrontier) {
-                    // its peg: g_x == v, and the other peg of the pair is peg ^ x
-                    const uint32_t src = ((U & k) ? 1u : 0u) | (((U >> 1) & k) ? 2u : 0u);
-                    uint64_t us = used[0];
-                    us = src == 1 ? used[1] : src == 2 ? used[2] : src == 3 ? used[3] : us;
-                    S &= ~us;
-                    if (!S) continue;
-                    children += __popcll(S);
-                    plane = src ^ uint32_t(x);
-                }
-                const uint32_t T = U ^ (k * uint32_t(x));
-                const uint32_t t = T - U0;
-                if (t < units) mark_local(MODE == kFrontier ? 4 * t + plane : t, S);
-                else mark_remote(T, S, plane);
+        // Larger disks, one per peg pair (x, v): the states S of the unit that
+        // move one, to unit T (frontier search: as operator `plane`).
+        auto pair = [&](uint32_t x, uint32_t v, uint64_t& S, uint32_t& T, uint32_t& plane) {
+            const uint32_t g = x == 1 ? U >> 1 : x == 2 ? U : U ^ (U >> 1);
+            const uint32_t e = (v ? g : ~g) & E;  // larger disks on the pair
+            const uint32_t k = e & (0u - e);      // the smallest of them
+            if (!k) {  // both pegs empty: no move
+                if constexpr (MODE != kFrontier) children -= __popcll(S);
+                S = 0;
             }
+            if constexpr (MODE == kFrontier) {
+                // its peg: g_x == v, and the other peg of the pair is peg ^ x
+                const uint32_t src = ((U & k) ? 1u : 0u) | (((U >> 1) & k) ? 2u : 0u);
+                S &= ~(src == 0 ? used[0] : src == 1 ? used[1] : src == 2 ? used[2] : used[3]);
+                plane = src ^ x;
+            }
+            T = U ^ (k * x);
+        };
+        uint32_t far_pairs = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < 6; ++i) {
+            uint64_t S = F & unit_free_mask<MODE>(1 + int(i >> 1), int(i & 1));
+            if (!S) continue;
+            uint32_t T, plane = 0;
+            pair(1 + (i >> 1), i & 1, S, T, plane);
+            if (!S) continue;
+            if constexpr (MODE == kFrontier) children += __popcll(S);
+            const uint32_t t = T - U0;
+            if (t < units) mark_local(MODE == kFrontier ? 4 * t + plane : t, S);
+            else far_pairs |= 1u << i;
+        }
+        // Moves that leave the window (under 1%), worked out again here: one
+        // copy of the long-range code instead of six.
+        while (far_pairs) {
+            const uint32_t i = __ffs(far_pairs) - 1;
+            far_pairs &= far_pairs - 1;
+            uint64_t S = F;
+#pragma unroll
+            for (uint32_t j = 0; j < 6; ++j)
+                if (j == i) S &= unit_free_mask<MODE>(1 + int(j >> 1), int(j & 1));
+            uint32_t T, plane = 0;
+            pair(1 + (i >> 1), i & 1, S, T, plane);
+            mark_remote(T, S, plane);
         }
     };
     auto expand_queued = [&](uint32_t i) {
@@ -275,123 +325,151 @@ __device__ __forceinline__ void hanoi_window(const LevelArgs& a, uint64_t window
     };
 
     constexpr int kWords = MODE == kTwoBit ? 2 : MODE == kFrontier ? 4 : 1;  // array words per unit
-    auto load = [&](uint32_t ch, uint64_t (&w)[kWords]) {
-        const uint32_t u = ch * 32 + uint32_t(lane);
+    // A warp sweeps groups of kGroup chunks (32 units each), all of whose
+    // words it loads at once; groups come from a shared counter.
+    constexpr int kGroup = hanoi_group(MODE);
+    uint32_t grp = uint32_t(warp), queued = 0;
+    for (bool more = grp * kGroup < chunks; more;) {  // uniform within the warp
+        uint64_t cw[kGroup][kWords];
 #pragma unroll
-        for (int q = 0; q < kWords; ++q) w[q] = 0;
-        if (ch >= chunks || u >= units) return;
-        const uint64_t* p = a.front + uint64_t(U0 + u) * kWords;
-        if constexpr (kWords == 1) {
-            w[0] = *p;
-        } else {
+        for (int c = 0; c < kGroup; ++c) {
+            const uint32_t u = (grp * kGroup + c) * 32 + uint32_t(lane);
 #pragma unroll
-            for (int q = 0; q < kWords; q += 2) {
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + q);
-                w[q] = v.x;
-                w[q + 1] = v.y;
-            }
-        }
-    };
-
-    uint64_t cw[kWords], nw[kWords];
-    uint32_t ch = uint32_t(warp), queued = 0;
-    load(ch, cw);
-    while (ch < chunks) {  // uniform within the warp
-        uint32_t nch = 0;
-        if (lane == 0) nch = atomicAdd(&sh.next_chunk, 1u);
-        nch = __shfl_sync(0xFFFFFFFFu, nch, 0);
-        load(nch, nw);
-        const uint32_t u = ch * 32 + uint32_t(lane);
-        uint64_t F[kPlanes] = {};
-        if constexpr (MODE == kTwoBit) {
-            uint64_t cur[2];
+            for (int q = 0; q < kWords; ++q) cw[c][q] = 0;
+            if (u >= units) continue;
+            const uint64_t* p = a.front + uint64_t(U0 + u) * kWords;
+            if constexpr (kWords == 1) {
+                cw[c][0] = *p;
+            } else {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint64_t hi = cw[h] & kEven, lo = (cw[h] >> 1) & kEven;
-                cur[h] = hi & (a.cur_code == 3 ? lo : ~lo);
-                if (cur[h])  // CUR -> OLD (code 1); only this block changes this window's CUR codes
-                    atomicXor(reinterpret_cast<unsigned long long*>(a.front) + 2ull * (U0 + u) + h,
-                              (unsigned long long)(cur[h] | (a.cur_code == 2 ? (cur[h] << 1) : 0)));
-            }
-            F[0] = cur[0] | (cur[1] << 1);
-            found += __popcll(F[0]);
-        } else if constexpr (MODE == kFrontier) {
-            if (cw[0] | cw[1] | cw[2] | cw[3]) {
-                uint64_t states = 0;  // in index order
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (cw[q]) a.front[4ull * (U0 + u) + q] = 0;  // FourBitArray::ScanAndClear
-                    states |= uint64_t(nibble_flags(cw[q])) << (16 * q);
-                }
-                uint64_t keep = states;
-                if (a.odd) {
-                    keep &= ~a.excl_cur[U0 + u];
-                    if (keep) a.excl_next[U0 + u] = keep;  // excl_next is clear before the level
-                }
-                found += __popcll(keep);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    // nibbles of the kept states of word q
-                    uint64_t k = (keep >> (16 * q)) & 0xFFFFull;
-                    k = (k | (k << 24)) & 0x000000FF000000FFull;
-                    k = (k | (k << 12)) & 0x000F000F000F000Full;
-                    k = (k | (k << 6)) & 0x0303030303030303ull;
-                    k = (k | (k << 3)) & 0x1111111111111111ull;
-#pragma unroll
-                    for (int p = 0; p < kPlanes; ++p) F[p] |= ((cw[q] >> p) & k) << q;
+                for (int q = 0; q < kWords; q += 2) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + q);
+                    cw[c][q] = v.x;
+                    cw[c][q + 1] = v.y;
                 }
             }
-        } else {
-            F[0] = cw[0];
-            if constexpr (MODE == kClassic) {
-                if (F[0]) a.front[U0 + u] = 0;  // BitArray::ScanBitsAndClear
-            }
-            found += __popcll(F[0]);
         }
-        uint64_t any = F[0];
+        uint32_t next = 0;
+        if (lane == 0) next = atomicAdd(&sh.next_chunk, 1u);
 #pragma unroll
-        for (int p = 1; p < kPlanes; ++p) any |= F[p];
-        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, any != 0);
-        if (any) {
-            const uint32_t at = queued + __popc(bal & ((1u << lane) - 1u));
-#pragma unroll
-            for (int p = 0; p < kPlanes; ++p) qmask[at * kPlanes + p] = F[p];
-            qunit[at] = uint16_t(u);
-        }
-        queued += __popc(bal);
-        __syncwarp();
-        if (queued >= 32) {
-            queued -= 32;
-            expand_queued(queued + uint32_t(lane));
-            __syncwarp();
-        }
-#pragma unroll
-        for (int q = 0; q < kWords; ++q) cw[q] = nw[q];
-        ch = nch;
-    }
-    if (uint32_t(lane) < queued) expand_queued(uint32_t(lane));
-    if (found != 0) sh.any = 1;
-    __syncthreads();
-
-    uint32_t fresh = 0;
-    if (sh.any) {
-        if (a.wflag_next && tid == 0) a.wflag_next[window] = 1;
-        for (uint32_t u = tid; u < units; u += KTHREADS) {
+        for (int c = 0; c < kGroup; ++c) {
+            const uint32_t u = (grp * kGroup + c) * 32 + uint32_t(lane);
+            uint64_t F[kPlanes] = {};
             if constexpr (MODE == kTwoBit) {
-                const uint64_t v = smem64[u];
-                if (!v) continue;
-                unsigned long long* codes = reinterpret_cast<unsigned long long*>(a.marks) + 2ull * (U0 + u);
-                const ulonglong2 w = __ldcg(reinterpret_cast<const ulonglong2*>(codes));
-                const uint64_t m0 = v & ~(w.x | (w.x >> 1)) & kEven;
-                const uint64_t m1 = (v >> 1) & ~(w.y | (w.y >> 1)) & kEven;
-                if (m0) atomicOr(codes, (unsigned long long)(m0 | ((next_pat & 2u) ? (m0 << 1) : 0)));
-                if (m1) atomicOr(codes + 1, (unsigned long long)(m1 | ((next_pat & 2u) ? (m1 << 1) : 0)));
-                fresh += __popcll(m0 | (m1 << 1));
-            } else if constexpr (MODE == kFrontier) {
+                const uint64_t flip = a.cur_code == 3 ? 0 : ~uint64_t(0);
+                const uint64_t c0 = cw[c][0] & ((cw[c][0] >> 1) ^ flip) & kEven;
+                const uint64_t c1 = cw[c][1] & ((cw[c][1] >> 1) ^ flip) & kEven;
+                F[0] = c0 | (c1 << 1);
+            } else {
+                F[0] = cw[c][0];
+                if constexpr (MODE == kFrontier) F[0] |= cw[c][1] | cw[c][2] | cw[c][3];
+            }
+            if (!__any_sync(0xFFFFFFFFu, F[0] != 0)) continue;  // nothing in these 32 units
+            if (F[0]) {
+                if constexpr (MODE == kTwoBit) {
+                    // CUR -> OLD (code 1); only this block changes this window's CUR codes
+                    unsigned long long* g = reinterpret_cast<unsigned long long*>(a.front) + 2ull * (U0 + u);
+                    const uint64_t c0 = F[0] & kEven, c1 = (F[0] >> 1) & kEven;
+                    if (c0) atomicXor(g, (unsigned long long)(c0 | (a.cur_code == 2 ? (c0 << 1) : 0)));
+                    if (c1) atomicXor(g + 1, (unsigned long long)(c1 | (a.cur_code == 2 ? (c1 << 1) : 0)));
+                } else if constexpr (MODE == kClassic) {
+                    a.front[U0 + u] = 0;  // BitArray::ScanBitsAndClear
+                } else if constexpr (MODE == kFrontier) {
+                    uint64_t keep = 0;  // in index order
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (cw[c][q]) a.front[4ull * (U0 + u) + q] = 0;  // FourBitArray::ScanAndClear
+                        keep |= uint64_t(nibble_flags(cw[c][q])) << (16 * q);
+                    }
+                    if (a.odd) {
+                        keep &= ~a.excl_cur[U0 + u];
+                        if (keep) a.excl_next[U0 + u] = keep;  // excl_next is clear before the level
+                    }
+                    found += __popcll(keep);
+#pragma unroll
+                    for (int p = 0; p < kPlanes; ++p) F[p] = 0;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        // nibbles of the kept states of word q
+                        uint64_t k = (keep >> (16 * q)) & 0xFFFFull;
+                        k = (k | (k << 24)) & 0x000000FF000000FFull;
+                        k = (k | (k << 12)) & 0x000F000F000F000Full;
+                        k = (k | (k << 6)) & 0x0303030303030303ull;
+                        k = (k | (k << 3)) & 0x1111111111111111ull;
+#pragma unroll
+                        for (int p = 0; p < kPlanes; ++p) F[p] |= ((cw[c][q] >> p) & k) << q;
+                    }
+                }
+                if constexpr (MODE != kFrontier) found += __popcll(F[0]);
+            }
+            uint64_t any = F[0];
+#pragma unroll
+            for (int p = 1; p < kPlanes; ++p) any |= F[p];
+            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, any != 0);
+            if (any) {
+                const uint32_t at = queued + __popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+                for (int p = 0; p < kPlanes; ++p) qmask[at * kPlanes + p] = F[p];
+                qunit[at] = uint16_t(u);
+            }
+            queued += __popc(bal);
+        }
+        grp = __shfl_sync(0xFFFFFFFFu, next, 0);
+        more = grp * kGroup < chunks;
+        __syncwarp();
+        // 32 units at a time; after the last group what is left.  The one
+        // place that expands: inlined twice it outgrows the instruction cache
+        // (17 disks two-bit: 250 ms with four copies, 140 ms with two).
+        while (queued >= (more ? 32u : 1u)) {
+            const uint32_t n = queued < 32 ? queued : 32u;
+            queued -= n;
+            if (uint32_t(lane) < n) expand_queued(queued + uint32_t(lane));
+        }
+        __syncwarp();
+    }
+    const bool any = __syncthreads_or(found != 0);
+    if (tid == 0) sh.next_chunk = kWarps;
+    uint32_t fresh = 0;
+    if (any) {  // flush the marks and clear them
+        if (a.wflag_next && tid == 0) a.wflag_next[window] = 1;
+        if constexpr (MODE == kTwoBit) {
+            // The codes were read by the sweep and mostly still sit in L1.  A
+            // stale word only lacks NEXT codes that other blocks set since,
+            // and setting those again changes nothing (`fresh` is an upper
+            // estimate).  Four units a turn keep four reads in flight.
+            ulonglong2* codes = reinterpret_cast<ulonglong2*>(a.marks) + U0;
+            for (uint32_t u0 = tid; u0 < units; u0 += 4 * KTHREADS) {
+                uint64_t v[4];
+                ulonglong2 w[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint32_t u = u0 + q * KTHREADS;
+                    v[q] = u < units ? smem64[u] : 0;
+                    if (v[q]) {
+                        w[q] = codes[u];
+                        smem64[u] = 0;
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (!v[q]) continue;
+                    unsigned long long* c = reinterpret_cast<unsigned long long*>(codes + u0 + q * KTHREADS);
+                    const uint64_t m0 = v[q] & ~(w[q].x | (w[q].x >> 1)) & kEven;
+                    const uint64_t m1 = (v[q] >> 1) & ~(w[q].y | (w[q].y >> 1)) & kEven;
+                    if (m0) atomicOr(c, (unsigned long long)(m0 | ((next_pat & 2u) ? (m0 << 1) : 0)));
+                    if (m1) atomicOr(c + 1, (unsigned long long)(m1 | ((next_pat & 2u) ? (m1 << 1) : 0)));
+                    fresh += __popcll(m0 | (m1 << 1));
+                }
+            }
+        }
+        for (uint32_t u = tid; MODE != kTwoBit && u < units; u += KTHREADS) {
+            if constexpr (MODE == kFrontier) {
                 uint64_t v[4];
 #pragma unroll
                 for (int p = 0; p < 4; ++p) v[p] = smem64[4 * u + p];
                 if (!(v[0] | v[1] | v[2] | v[3])) continue;
+#pragma unroll
+                for (int p = 0; p < 4; ++p) smem64[4 * u + p] = 0;
                 unsigned long long* g = reinterpret_cast<unsigned long long*>(a.marks) + 4ull * (U0 + u);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -402,31 +480,19 @@ __device__ __forceinline__ void hanoi_window(const LevelArgs& a, uint64_t window
                 }
             } else {
                 const unsigned long long v = smem64[u];
-                if (v) atomicOr(reinterpret_cast<unsigned long long*>(a.marks) + U0 + u, v);
+                if (!v) continue;
+                smem64[u] = 0;
+                atomicOr(reinterpret_cast<unsigned long long*>(a.marks) + U0 + u, v);
             }
         }
     }
 
-    const uint32_t c0 = __reduce_add_sync(0xFFFFFFFFu, found);
-    const uint32_t c1 = __reduce_add_sync(0xFFFFFFFFu, children);
-    const uint32_t c2 = __reduce_add_sync(0xFFFFFFFFu, children - remote);
-    uint32_t c5 = 0, c6 = 0;
-    if constexpr (MODE == kTwoBit) {
-        c5 = __reduce_add_sync(0xFFFFFFFFu, marked + fresh);
-        c6 = __reduce_add_sync(0xFFFFFFFFu, farmarks);
-    }
-    if (lane == 0) {
-        if (c0) atomicAdd(&sh.cnt[0], (unsigned long long)c0);
-        if (c1) atomicAdd(&sh.cnt[1], (unsigned long long)c1);
-        if (c2) atomicAdd(&sh.cnt[2], (unsigned long long)c2);
-        if (c5) atomicAdd(&sh.cnt[5], (unsigned long long)c5);
-        if (c6) atomicAdd(&sh.cnt[6], (unsigned long long)c6);
-    }
-    __syncthreads();  // the shared marks and queues may be reused for another window
-    if (tid == 0) {
-        for (int i = 0; i < 8; ++i)
-            if (sh.cnt[i]) atomicAdd(&a.stats[i], sh.cnt[i]);
-    }
+    __syncthreads();  // the marks are clear and the queues free
+    cnt.found += found;
+    cnt.children += children;
+    cnt.remote += remote;
+    cnt.next += marked + fresh;
+    cnt.farmarks += farmarks;
 }
 
 }  // namespace psb

@@ -980,12 +980,17 @@ size_t smem_bytes(int mode, int wb, int threads = 0) {
 // threads = 0, two-bit pancake and Hanoi searches of 2^32 states or more take
 // 128-thread blocks, five per SM (B200 sweeps, whole search, far marks NEAR:
 // 14-pancake 4.06 s at 128 threads vs 4.40 s at 256; 13-pancake 213 vs
-// 219 ms; 18-disk Hanoi 1.58 vs 1.77 s).  Three-bit (13-pancake 195 vs
-// 193 ms) and the sliding-tile puzzles (3x4 two-bit 45 vs 40 ms) keep 256.
+// 219 ms; symmetric 18-disk Hanoi).  Two-bit Hanoi without symmetry (64
+// states at a time, psb_hanoi_words.cuh) takes them at any size: a window's
+// warps finish closer together (17 disks 102 vs 109 ms).  Three-bit
+// (13-pancake 195 vs 193 ms) and the sliding-tile puzzles (3x4 two-bit 45 vs
+// 40 ms) keep 256.
 int shape_variant(const psb_puzzle* p, int mode, int threads) {
     if (mode != psb::kTwoBit && mode != psb::kThreeBit) return 0;
+    const bool hanoi = p->kind == PSB_HANOI4 || p->kind == PSB_HANOI4_OPT;
+    if (threads == 0 && mode == psb::kTwoBit && hanoi && !p->pz.sym) return 2;
     if (threads == 0 && mode == psb::kTwoBit && p->n_states >= (uint64_t(1) << 32) &&
-        (p->kind == PSB_PANCAKE || p->kind == PSB_PANCAKE_OPT || p->kind == PSB_HANOI4 || p->kind == PSB_HANOI4_OPT))
+        (hanoi || p->kind == PSB_PANCAKE || p->kind == PSB_PANCAKE_OPT))
         return 2;
     return threads == 512 ? 1 : threads == 128 ? 2 : 0;
 }
