@@ -780,6 +780,16 @@ int session_pool(int device, cudaMemPool_t* out) {
     return PSB_OK;
 }
 
+}  // namespace
+
+int psb::scratch_pool(cudaMemPool_t* pool) {
+    int device = 0;
+    PSB_CUDA(cudaGetDevice(&device));
+    return session_pool(device, pool);
+}
+
+namespace {
+
 // Frontier spill resources: the segment encoder (its device scratch), one
 // segment's extracted bitmap, an arena holding one depth's encoded segments
 // back to back, a copy stream and two pinned host slots.  A depth is encoded

@@ -122,7 +122,6 @@ struct Run {
     DevBuf<uint64_t> next, cur, old, kids;
     DevBuf<uint32_t> offs;
     DevBuf<uint8_t> stream_buf[2];  // the two layers decoded for one segment
-    DevBuf<psb_codec_block> block_tab[2];
     DevBuf<unsigned int> hist;
     DevBuf<unsigned long long> scalars;  // [0] count, [1] children appended, [2] error flag, [3] decode error
     psb::SegmentEncoder* enc = nullptr;  // device scratch kept from segment to segment
@@ -138,8 +137,10 @@ struct Run {
     psb_segmented_stats st{};
 
     ~Run() {
+        if (s) cudaStreamSynchronize(s);
         if (enc) psb::encoder_destroy(enc);
-        if (dec) psb::decoder_destroy(dec);
+        if (dec) psb::decoder_destroy(dec);  // frees its scratch in stream order
+        if (s) cudaStreamDestroy(s);
     }
 
     uint64_t states_in(uint64_t g) const { return std::min(seg_states, P->n_states - g * seg_states); }
@@ -162,14 +163,11 @@ struct Run {
         blocks.resize(nb);
         if (int rc = psb_frontier_index(host_stream.data(), bytes, blocks.data(), nb, &nb)) return rc;
         if (int rc = stream_buf[slot].grow(bytes)) return rc;
-        if (int rc = block_tab[slot].grow(nb)) return rc;
-        // Pageable sources: both copies have left host memory when the calls return.
+        // Pageable source: the copy has left host memory when the call returns.
         SG_CUDA(cudaMemcpyAsync(stream_buf[slot].p, host_stream.data(), bytes, cudaMemcpyHostToDevice, s));
-        SG_CUDA(cudaMemcpyAsync(block_tab[slot].p, blocks.data(), nb * sizeof(psb_codec_block),
-                                cudaMemcpyHostToDevice, s));
         st.h2d_bytes += bytes;
-        return psb::frontier_decode_async(stream_buf[slot].p, host_stream.data(), blocks.data(), block_tab[slot].p,
-                                          nb, bits, states_in(g), scalars.p + 3, dec, s);
+        return psb::frontier_decode_async(stream_buf[slot].p, blocks.data(), nb, bits, states_in(g), scalars.p + 3,
+                                          dec, s);
     }
 
     // Encodes a segment bitmap holding `count` states as segment g's layer in `store`.
@@ -354,7 +352,6 @@ extern "C" int psb_bfs_segmented(const psb_puzzle* p, uint64_t initial, const ps
     };
 
     SG_CUDA(cudaStreamCreateWithFlags(&R.s, cudaStreamNonBlocking));
-    struct StreamGuard { cudaStream_t s; ~StreamGuard() { cudaStreamSynchronize(s); cudaStreamDestroy(s); } } guard{R.s};
     for (auto* b : {&R.next, &R.cur, &R.old})
         if (int rc = b->grow(R.seg_words)) return rc;
     if (int rc = R.kids.grow(R.chunk_words * 64 * uint64_t(p->branching))) return rc;
