@@ -36,7 +36,7 @@
 
 namespace psb {
 
-constexpr int kThreads = 256;  // finalize and batched-expand kernels
+constexpr int kThreads = 256;  // finalize kernels and the segment expansion
 
 enum Mode : int { kThreeBit = 0, kClassic = 1, kTwoBit = 2, kFrontier = 3 };
 
@@ -1073,7 +1073,12 @@ __global__ void seed_kernel(LevelArgs a, uint64_t initial) {
 // Batched Expand (Puzzle::Expand; GPU twin of Puzzles/PuzzleGpu.cpp:53-82):
 // one thread per parent, BranchingFactor slots per parent, valid children
 // first in the reference order, unused slots INVALID_INDEX with operator
-// (1 << OperatorsCount) - 1.
+// (1 << OperatorsCount) - 1.  A thread's slots are 12 bytes x BranchingFactor
+// apart from its neighbour's, so each warp puts its 32 parents' slots into
+// shared memory (rows of an odd number of slots: no bank conflicts) and
+// writes them out in order, 32 neighbouring slots per store.
+constexpr int kExpandThreads = 128;
+
 template <class PZ>
 struct SlotEmitter {
     uint64_t* out;
@@ -1087,29 +1092,42 @@ struct SlotEmitter {
 };
 
 template <class PZ, bool kOpBits>
-__global__ void __launch_bounds__(kThreads) expand_batch_kernel(const uint64_t* __restrict__ parents,
+__global__ void __launch_bounds__(kExpandThreads) expand_batch_kernel(const uint64_t* __restrict__ parents,
                                                                const uint32_t* __restrict__ opbits, uint64_t n,
                                                                uint64_t n_states, uint64_t* __restrict__ children,
                                                                uint32_t* __restrict__ child_ops, PuzzleArgs pz,
                                                                unsigned long long* err) {
-    const uint64_t i = blockIdx.x * uint64_t(kThreads) + threadIdx.x;
-    if (i >= n) return;
-    constexpr int kB = PZ::kBranch;
-    uint64_t* out = children + i * kB;
-    uint32_t* ops = child_ops + i * kB;
-    const uint64_t p = parents[i];
-    int k = 0;
-    if (p < n_states) {
-        SlotEmitter<PZ> em{out, ops};
-        PZ::template expand<kOpBits>(p, kOpBits ? opbits[i] : 0u, pz, em);
-        k = em.k;
-    } else {
-        atomicOr(err, 1ull);
+    constexpr int kB = PZ::kBranch, kRow = kB | 1;
+    __shared__ uint64_t s_out[kExpandThreads * kRow];
+    __shared__ uint32_t s_ops[kExpandThreads * kRow];
+    const uint32_t lane = threadIdx.x & 31u, first = threadIdx.x - lane;
+    const uint64_t i = blockIdx.x * uint64_t(kExpandThreads) + threadIdx.x;
+    if (i < n) {
+        uint64_t* out = s_out + threadIdx.x * kRow;
+        uint32_t* ops = s_ops + threadIdx.x * kRow;
+        const uint64_t p = parents[i];
+        int k = 0;
+        if (p < n_states) {
+            SlotEmitter<PZ> em{out, ops};
+            PZ::template expand<kOpBits>(p, kOpBits ? opbits[i] : 0u, pz, em);
+            k = em.k;
+        } else {
+            atomicOr(err, 1ull);
+        }
+        const uint32_t inv_op = (1u << PZ::kOps) - 1u;
+        for (; k < kB; ++k) {
+            out[k] = kInvalidIndex;
+            ops[k] = inv_op;
+        }
     }
-    const uint32_t inv_op = (1u << PZ::kOps) - 1u;
-    for (; k < kB; ++k) {
-        out[k] = kInvalidIndex;
-        ops[k] = inv_op;
+    __syncwarp();
+    const uint64_t base = i - lane;  // the warp's first parent
+    if (base >= n) return;
+    const uint32_t slots = uint32_t(n - base < 32 ? n - base : 32) * kB;
+    for (uint32_t j = lane; j < slots; j += 32) {
+        const uint32_t at = (first + j / kB) * kRow + j % kB;
+        children[base * kB + j] = s_out[at];
+        child_ops[base * kB + j] = s_ops[at];
     }
 }
 
@@ -1259,13 +1277,13 @@ cudaError_t launch_expand(const uint64_t* parents, const uint32_t* opbits, uint6
                           uint64_t* children, uint32_t* child_ops, PuzzleArgs pz, unsigned long long* err,
                           bool use_opbits, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    const unsigned grid = unsigned((n + kThreads - 1) / kThreads);
+    const unsigned grid = unsigned((n + kExpandThreads - 1) / kExpandThreads);
     if (use_opbits)
-        expand_batch_kernel<PZ, true><<<grid, kThreads, 0, s>>>(parents, opbits, n, n_states, children, child_ops,
-                                                                pz, err);
+        expand_batch_kernel<PZ, true><<<grid, kExpandThreads, 0, s>>>(parents, opbits, n, n_states, children,
+                                                                      child_ops, pz, err);
     else
-        expand_batch_kernel<PZ, false><<<grid, kThreads, 0, s>>>(parents, opbits, n, n_states, children, child_ops,
-                                                                 pz, err);
+        expand_batch_kernel<PZ, false><<<grid, kExpandThreads, 0, s>>>(parents, opbits, n, n_states, children,
+                                                                       child_ops, pz, err);
     return cudaGetLastError();
 }
 
