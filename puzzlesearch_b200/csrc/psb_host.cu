@@ -891,6 +891,7 @@ struct psb_bfs_session {
     uint64_t* visited = nullptr;  // three-bit searches that may run bottom-up: states at depth <= current
     uint32_t* far = nullptr;      // two-bit: long-range mark bitmap (1 bit per state), folded after each level
     uint64_t far_words = 0;       // its size in 64-bit words (padded)
+    bool own_windows = false;     // window_bits was not asked for (LevelArgs::own_windows)
     bool bottom_up = false;       // this search's algorithm and puzzle support bottom-up levels
     unsigned long long* d_stats = nullptr;
     unsigned long long* h_stats = nullptr;
@@ -1228,6 +1229,7 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
     LevelArgs a{};
     a.n_states = N;
     a.window_bits = S->window_bits;
+    a.own_windows = S->own_windows ? 1 : 0;
     a.odd = P.odd;
     a.pz = P.pz;
     a.stats = S->d_stats;
@@ -1575,6 +1577,7 @@ int psb_bfs_session_create(const psb_puzzle* p, int algo, const psb_bfs_opts* op
     if (int rc = ensure_device(S->device)) return rc;
     if (S->device < 0) PSB_CUDA(cudaGetDevice(&S->device));
     S->window_bits = (opts && opts->window_bits) ? opts->window_bits : auto_window_bits(p, algo);
+    S->own_windows = !(opts && opts->window_bits);
     if (S->window_bits < 10 || S->window_bits > 20 || (algo == PSB_FRONTIER && S->window_bits > 18))
         return fail(PSB_ERR_ARG, "window_bits %d out of range", S->window_bits);
     if (((p->n_states + (uint64_t(1) << S->window_bits) - 1) >> S->window_bits) > 0x7FFFFFFFull)

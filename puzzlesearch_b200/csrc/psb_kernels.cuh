@@ -271,6 +271,8 @@ struct LevelArgs {
     int sym_mult;               // Hanoi with symmetry: add each frontier state's class size to stats[7]
     int flag_bits;              // non-zero: wflag_next has one byte per 2^flag_bits states (a bottom-up level's
                                 // windows are larger than the top-down windows its flags serve); 0: window_bits
+    int own_windows;            // window_bits was not asked for: a top-down kernel with windows of its own shape may
+                                // use them (the flags stay one byte per 2^window_bits states)
 };
 
 constexpr uint64_t kEven = 0x5555555555555555ull;

@@ -151,6 +151,7 @@ extern "C" int psb_bfs_noalloc(const psb_puzzle* p, int algo, uint64_t initial, 
     psb::LevelArgs a{};
     a.n_states = N;
     a.window_bits = wb;
+    a.own_windows = 1;
     a.odd = p->odd;
     a.pz = p->pz;
     a.stats = d_stats;

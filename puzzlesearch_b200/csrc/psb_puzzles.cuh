@@ -78,27 +78,13 @@ __host__ __device__ constexpr uint64_t fact(int k) {
 }
 constexpr uint32_t kF12 = 479001600u;  // 12!
 
-// Lehmer digits of a permutation index.  Digits with weight < 12! come from
-// the low 32-bit part; the (at most four) top digits of n > 12 from the quotient.
+// Lehmer digits of a permutation index below 2^32.
 template <int N>
-__device__ __forceinline__ void perm_digits(uint64_t index, uint32_t (&d)[N]) {
-    uint32_t lo, hi = 0;
-    if constexpr (N <= 12) {
-        lo = uint32_t(index);
-    } else {
-        hi = uint32_t(index / kF12);
-        lo = uint32_t(index - uint64_t(hi) * kF12);
-    }
+__device__ __forceinline__ void perm_digits(uint32_t index, uint32_t (&d)[N]) {
 #pragma unroll
     for (int i = N - 1; i >= 0; --i) {
-        const uint32_t radix = uint32_t(N - i);
-        if (N - 1 - i < 12) {
-            d[i] = lo % radix;
-            lo /= radix;
-        } else {
-            d[i] = hi % radix;
-            hi /= radix;
-        }
+        d[i] = index % uint32_t(N - i);
+        index /= uint32_t(N - i);
     }
 }
 
@@ -124,92 +110,74 @@ __device__ __forceinline__ void perm_values(const uint32_t (&d)[N], uint32_t (&v
 // low_m(child) = sum_{q<m} q! * #(earlier values of the parent suffix that
 // are smaller than the parent value at position n-m+q).
 // --------------------------------------------------------------------------
+
+// n > 7.  The first kL = n-7 positions of an index depend on index / 7! only
+// (digit i has weight (n-1-i)!): every index of a block of 7! = 5040 shares
+// them, and their part of each larger flip's rank is a constant of the block.
+// A Prefix holds those constants; a state unranks its last seven values from
+// index % 7! and adds their terms: 60 popcounts a parent at 13 pancakes
+// instead of 75, no digits or masks of the other positions, and 70 registers
+// instead of 96 to 128.
+// (A table of the 5040 arrangements, with or without the small flips'
+// deltas, instead of the unranking: no faster, 132.8 to 134.0 against
+// 135.0 ms; its loads queue behind the marks.)
 template <int N>
-struct Pancake {
+struct PancakeLarge {
     static constexpr int kBranch = N - 1;
     static constexpr int kOps = N - 1;
-
-    // Chunk-shared unranking.  Digit i has weight (n-1-i)!, so the first
-    // kL = n-7 positions of an index depend only on index / 7!: every index
-    // of a block of 7! = 5040 consecutive indexes shares them.  A Prefix holds
-    // those positions (digits, pre, pb) and the other 7 values as a 32-bit
-    // nibble list; unrank_suffix completes a state from index % 7!.
-    static constexpr int kL = N > 7 ? N - 7 : 0;
+    static constexpr int kL = N - 7;
     static constexpr uint32_t kBlock = 5040;  // 7!
+    static constexpr int kNear = (N < 12 ? N : 12) - 7;  // flips of 8 .. 12
+    static constexpr int kFar = N > 12 ? N - 12 : 1;     // flips of 13 ..
     struct Prefix {
-        uint32_t d[kL > 0 ? kL : 1], pre[kL > 0 ? kL : 1], pb[kL > 0 ? kL : 1];
         uint32_t acc;     // values at positions < kL, one bit each
         uint32_t tiles7;  // the other 7 values, ascending, one nibble each
+        struct {
+            uint32_t base;  // of flip m: (terms of the positions < kL) - (their parent digits), mod 2^32
+            uint32_t keep;  // values not left of the flip
+        } near[kNear];
+        uint32_t far_keep[kFar];
+        uint64_t far_base[kFar];
     };
-
-    // Lehmer digits d, and for each position j: pre[j] = values left of j,
-    // pb[j] = those of them smaller than v[j] (one bit per value).
-    __device__ __forceinline__ static void unrank(uint64_t index, uint32_t (&d)[N], uint32_t (&pre)[N],
-                                                  uint32_t (&pb)[N]) {
-        uint32_t v[N];
-        perm_digits<N>(index, d);
-        perm_values<N>(d, v);
-        uint32_t acc = 0;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            pre[i] = acc;
-            pb[i] = acc & ((1u << v[i]) - 1u);
-            acc |= 1u << v[i];
-        }
-    }
 
     // Prefix of the indexes in [q*7!, (q+1)*7!); q < n!/7! <= 16!/7! < 2^32.
     __device__ __forceinline__ static void make_prefix(uint32_t q, Prefix& P) {
-        if constexpr (kL > 0) {
-            uint32_t d[kL];
+        uint32_t d[kL], pre[kL], pb[kL];  // digits; values left of the position; those smaller than its own
 #pragma unroll
-            for (int i = kL - 1; i >= 0; --i) {
-                d[i] = q % uint32_t(N - i);
-                q /= uint32_t(N - i);
-            }
-            uint64_t tiles = 0xFEDCBA9876543210ull;
-            uint32_t acc = 0;
-#pragma unroll
-            for (int i = 0; i < kL; ++i) {
-                const uint32_t s = 4u * d[i];
-                const uint32_t v = uint32_t(tiles >> s) & 15u;
-                tiles = (((tiles >> s) >> 4) << s) | (tiles & ((uint64_t(1) << s) - 1));
-                P.d[i] = d[i];
-                P.pre[i] = acc;
-                P.pb[i] = acc & ((1u << v) - 1u);
-                acc |= 1u << v;
-            }
-            P.acc = acc;
-            P.tiles7 = uint32_t(tiles) & 0x0FFFFFFFu;
-        } else {
-            P.acc = 0;
-            P.tiles7 = 0x06543210u;
+        for (int i = kL - 1; i >= 0; --i) {
+            d[i] = q % uint32_t(N - i);
+            q /= uint32_t(N - i);
         }
-    }
-
-    // State of index q*7! + r from its block's prefix (r < 7!).
-    __device__ __forceinline__ static void unrank_suffix(const Prefix& P, uint32_t r, uint32_t (&d)[N],
-                                                         uint32_t (&pre)[N], uint32_t (&pb)[N]) {
+        uint64_t tiles = 0xFEDCBA9876543210ull;
+        uint32_t acc = 0;
 #pragma unroll
         for (int i = 0; i < kL; ++i) {
-            d[i] = P.d[i];
-            pre[i] = P.pre[i];
-            pb[i] = P.pb[i];
-        }
-#pragma unroll
-        for (int i = N - 1; i >= kL; --i) {
-            d[i] = r % uint32_t(N - i);
-            r /= uint32_t(N - i);
-        }
-        uint32_t t = P.tiles7, acc = P.acc;
-#pragma unroll
-        for (int i = kL; i < N; ++i) {
             const uint32_t s = 4u * d[i];
-            const uint32_t v = (t >> s) & 15u;
-            t = ((t >> s) >> 4 << s) | (t & ((1u << s) - 1u));
+            const uint32_t v = uint32_t(tiles >> s) & 15u;
+            tiles = (((tiles >> s) >> 4) << s) | (tiles & ((uint64_t(1) << s) - 1));
             pre[i] = acc;
             pb[i] = acc & ((1u << v) - 1u);
             acc |= 1u << v;
+        }
+        P.acc = acc;
+        P.tiles7 = uint32_t(tiles) & 0x0FFFFFFFu;
+#pragma unroll
+        for (int m = 8; m <= N; ++m) {
+            const int i = N - m;
+            uint64_t base = 0;
+#pragma unroll
+            for (int j = i; j < kL; ++j) {
+                const uint32_t c = j > i ? __popc(pb[j] & ~pre[i]) : 0;
+                if (m <= 12) base = uint32_t(base) + uint32_t(fact(j - i)) * c - d[j] * uint32_t(fact(N - 1 - j));
+                else base += fact(j - i) * c - uint64_t(d[j]) * fact(N - 1 - j);
+            }
+            if (m <= 12) {
+                P.near[m - 8].base = uint32_t(base);
+                P.near[m - 8].keep = ~pre[i];
+            } else {
+                P.far_base[m - 13 < kFar ? m - 13 : 0] = base;
+                P.far_keep[m - 13 < kFar ? m - 13 : 0] = ~pre[i];
+            }
         }
     }
 
@@ -222,96 +190,148 @@ struct Pancake {
     template <bool kOpBits, class Emit>
     __device__ __forceinline__ static void expand_range(uint64_t index, uint32_t opbits, int first, int last,
                                                         Emit& emit) {
-        uint32_t d[N], pre[N], pb[N];
-        unrank(index, d, pre, pb);
-        children<kOpBits>(index, d, pre, pb, opbits, first, last, emit);
+        const uint32_t q = uint32_t(index / kBlock);
+        Prefix P;
+        make_prefix(q, P);
+        expand_prefixed<kOpBits>(index, P, uint32_t(index - uint64_t(q) * kBlock), opbits, first, last, emit);
     }
 
-    // expand_range for index = q*7! + r, with P = make_prefix(q).
-    template <bool kOpBits, class Emit>
-    __device__ __forceinline__ static void expand_prefixed(uint64_t index, const Prefix& P, uint32_t r,
-                                                           uint32_t opbits, int first, int last, Emit& emit) {
-        uint32_t d[N], pre[N], pb[N];
-        unrank_suffix(P, r, d, pre, pb);
-        children<kOpBits>(index, d, pre, pb, opbits, first, last, emit);
-    }
-
-    // Rank of the child of flip m: with pre = the values left of the suffix
-    // (positions < n-m) and pb[j] = the values left of position j that are
-    // smaller than v[j], the count above is popc(pb[j] & ~pre).  For m <= 12
+    // expand_range for index = q*7! + r, with P = make_prefix(q).  For m <= 12
     // every quantity is below 12! < 2^31, so the child is passed to emitters
     // that take it (EmitRel) as the parent plus a 32-bit signed delta.
     template <bool kOpBits, class Emit>
-    __device__ __forceinline__ static void children(uint64_t index, const uint32_t (&d)[N], const uint32_t (&pre)[N],
-                                                    const uint32_t (&pb)[N], uint32_t opbits, int first, int last,
-                                                    Emit& emit) {
+    __device__ __forceinline__ static void expand_prefixed(uint64_t index, const Prefix& prefix, uint32_t r,
+                                                           uint32_t opbits, int first, int last, Emit& emit) {
+        const Prefix P = prefix;  // in registers: marks may alias a prefix in shared memory
+        // pb[t]: the values left of the t-th of the last seven that are smaller
+        // and pre[t] those left of it at all
+        uint32_t d[7], pb[7], pre[7], low[7], acc = P.acc, tiles7 = P.tiles7;
+        uint32_t x = r;
+#pragma unroll
+        for (int t = 6; t >= 0; --t) {
+            d[t] = x % uint32_t(7 - t);
+            x /= uint32_t(7 - t);
+            low[t] = r - x * uint32_t(fact(7 - t));  // r mod (7-t)!
+        }
+#pragma unroll
+        for (int t = 0; t < 7; ++t) {
+            const uint32_t s = 4u * d[t];
+            const uint32_t bit = 1u << ((tiles7 >> s) & 15u);
+            tiles7 = ((tiles7 >> s) >> 4 << s) | (tiles7 & ((1u << s) - 1u));
+            pre[t] = acc;
+            pb[t] = acc & (bit - 1u);
+            acc |= bit;
+        }
+        auto skip = [&](int op) { return op < first || op >= last || (kOpBits && ((opbits >> op) & 1u)); };
+        auto far_child = [&](int m) -> uint64_t {  // m >= 13
+            const uint32_t keep = P.far_keep[m - 13 < kFar ? m - 13 : 0];
+            uint32_t s32 = 0, hi = 0;
+#pragma unroll
+            for (int t = 0; t < 7; ++t) {
+                const uint32_t c = __popc(pb[t] & keep);
+                if (m - 7 + t < 12) s32 += uint32_t(fact(m - 7 + t)) * c;
+                else hi += uint32_t(fact(m - 7 + t) / kF12) * c;
+            }
+            return index + P.far_base[m - 13 < kFar ? m - 13 : 0] - r + (uint64_t(hi) * kF12 + s32);
+        };
         // Far children first, for emitters that take them in two steps.
         constexpr bool kSplit = EmitSplitFar<Emit>::value && (N > 12);
-        constexpr int kFarN = N > 12 ? N - 12 : 1;
-        uint64_t far_child[kFarN];
-        FarTicket far_ticket[kFarN];
+        uint64_t far[kFar];
+        FarTicket ticket[kFar];
         if constexpr (kSplit) {
-            uint64_t low = 0;
 #pragma unroll
-            for (int m = 2; m <= N; ++m) {
-                low += uint64_t(d[N - m]) * fact(m - 1);
-                if (m <= 12) continue;
-                const int op = m - 2, k = m - 13;
-                far_ticket[k].pending = false;
-                if (op < first || op >= last || (kOpBits && (opbits >> op) & 1u)) {
-                    far_child[k] = kInvalidIndex;
-                    continue;
-                }
-                const uint32_t excl = pre[N - m];
-                uint32_t s32 = 0, t = 0;
-#pragma unroll
-                for (int q = 1; q < m; ++q) {
-                    const uint32_t c = __popc(pb[N - m + q] & ~excl);
-                    if (q < 12) s32 += uint32_t(fact(q)) * c;
-                    else t += uint32_t(fact(q) / kF12) * c;
-                }
-                far_child[k] = index - low + (uint64_t(t) * kF12 + s32);
-                far_ticket[k] = emit.far_issue(far_child[k], uint32_t(op));
+            for (int m = 13; m <= N; ++m) {
+                far[m - 13] = kInvalidIndex;
+                if (skip(m - 2)) continue;
+                far[m - 13] = far_child(m);
+                ticket[m - 13] = emit.far_issue(far[m - 13], uint32_t(m - 2));
             }
         }
-        uint32_t low32 = 0;  // low_m for m <= 12 (d[n-1] is always 0)
-        uint64_t low64 = 0;  // low_m for m > 12
 #pragma unroll
         for (int m = 2; m <= N; ++m) {
-            if (kSplit && m > 12) break;
-            if (m <= 12) low32 += d[N - m] * uint32_t(fact(m - 1));
-            else low64 = (m == 13 ? uint64_t(low32) : low64) + uint64_t(d[N - m]) * fact(m - 1);
-            const int op = m - 2;
-            if (op >= last) break;
-            if (op < first || (kOpBits && (opbits >> op) & 1u)) continue;
-            const uint32_t excl = pre[N - m];
+            if (skip(m - 2)) continue;
             if (m <= 12) {  // m is a compile-time constant after unrolling
-                uint32_t s32 = 0;
+                int32_t delta;
+                if (m <= 7) {
+                    const int t0 = 7 - m;
+                    uint32_t s32 = 0;
 #pragma unroll
-                for (int q = 1; q < m; ++q) s32 += uint32_t(fact(q)) * __popc(pb[N - m + q] & ~excl);
-                const int32_t delta = int32_t(s32 - low32);
-                if constexpr (EmitRel<Emit>::value) emit.rel(index, delta, uint32_t(op));
-                else emit(index + int64_t(delta), uint32_t(op));
-            } else {
-                uint32_t s32 = 0, t = 0;
+                    for (int t = t0 + 1; t < 7; ++t) s32 += uint32_t(fact(t - t0)) * __popc(pb[t] & ~pre[t0]);
+                    delta = int32_t(s32 - low[t0]);
+                } else {
+                    const auto f = P.near[m - 8 < kNear ? m - 8 : 0];
+                    uint32_t s32 = f.base - r;
 #pragma unroll
-                for (int q = 1; q < m; ++q) {
-                    const uint32_t c = __popc(pb[N - m + q] & ~excl);
-                    if (q < 12) s32 += uint32_t(fact(q)) * c;
-                    else t += uint32_t(fact(q) / kF12) * c;
+                    for (int t = 0; t < 7; ++t) s32 += uint32_t(fact(m - 7 + t)) * __popc(pb[t] & f.keep);
+                    delta = int32_t(s32);
                 }
-                const uint64_t child = index - low64 + (uint64_t(t) * kF12 + s32);
-                if constexpr (EmitFar<Emit>::value) emit.far(child, uint32_t(op));
-                else emit(child, uint32_t(op));
+                if constexpr (EmitRel<Emit>::value) emit.rel(index, delta, uint32_t(m - 2));
+                else emit(index + int64_t(delta), uint32_t(m - 2));
+            } else if (!kSplit) {
+                const uint64_t child = far_child(m);
+                if constexpr (EmitFar<Emit>::value) emit.far(child, uint32_t(m - 2));
+                else emit(child, uint32_t(m - 2));
             }
         }
         if constexpr (kSplit) {
 #pragma unroll
             for (int k = 0; k < N - 12; ++k)
-                if (far_child[k] != kInvalidIndex) emit.far_finish(far_child[k], uint32_t(k + 11), far_ticket[k]);
+                if (far[k] != kInvalidIndex) emit.far_finish(far[k], uint32_t(k + 11), ticket[k]);
         }
     }
 };
+
+// n <= 7: one block of at most 7! indexes.
+template <int N>
+struct PancakeSmall {
+    static constexpr int kBranch = N - 1;
+    static constexpr int kOps = N - 1;
+    static constexpr uint32_t kBlock = 5040;
+    struct Prefix { uint32_t unused; };
+    __device__ __forceinline__ static void make_prefix(uint32_t, Prefix&) {}
+
+    template <bool kOpBits, class Emit>
+    __device__ __forceinline__ static void expand(uint64_t index, uint32_t opbits, Emit& emit) {
+        expand_range<kOpBits>(index, opbits, 0, N - 1, emit);
+    }
+    template <bool kOpBits, class Emit>
+    __device__ __forceinline__ static void expand_prefixed(uint64_t index, const Prefix&, uint32_t, uint32_t opbits,
+                                                           int first, int last, Emit& emit) {
+        expand_range<kOpBits>(index, opbits, first, last, emit);
+    }
+    // Rank of the child of flip m: with pre = the values left of the suffix
+    // (positions < n-m) and pb[j] = the values left of position j that are
+    // smaller than v[j], the count above is popc(pb[j] & ~pre).
+    template <bool kOpBits, class Emit>
+    __device__ __forceinline__ static void expand_range(uint64_t index, uint32_t opbits, int first, int last,
+                                                        Emit& emit) {
+        uint32_t d[N], v[N], pre[N], pb[N];
+        perm_digits<N>(uint32_t(index), d);
+        perm_values<N>(d, v);
+        uint32_t acc = 0;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            pre[i] = acc;
+            pb[i] = acc & ((1u << v[i]) - 1u);
+            acc |= 1u << v[i];
+        }
+        uint32_t low = 0;  // low_m (d[n-1] is always 0)
+#pragma unroll
+        for (int m = 2; m <= N; ++m) {
+            low += d[N - m] * uint32_t(fact(m - 1));
+            const int op = m - 2;
+            if (op < first || op >= last || (kOpBits && ((opbits >> op) & 1u))) continue;
+            uint32_t s = 0;
+#pragma unroll
+            for (int q = 1; q < m; ++q) s += uint32_t(fact(q)) * __popc(pb[N - m + q] & ~pre[N - m]);
+            const int32_t delta = int32_t(s - low);
+            if constexpr (EmitRel<Emit>::value) emit.rel(index, delta, uint32_t(op));
+            else emit(index + int64_t(delta), uint32_t(op));
+        }
+    }
+};
+template <int N>
+using Pancake = typename std::conditional<(N > 7), PancakeLarge<(N > 7 ? N : 8)>, PancakeSmall<(N > 7 ? 7 : N)>>::type;
 
 // --------------------------------------------------------------------------
 // Sliding tile (SlidingTilePuzzleSimple.cpp:8,61-99): operators UP=0, LEFT=1,
