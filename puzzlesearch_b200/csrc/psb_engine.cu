@@ -34,6 +34,7 @@
 #include "../../include/psb200.h"
 #include "psb_hanoi_words.cuh"
 #include "psb_internal.h"
+#include "psb_pancake_windows.cuh"
 
 namespace psb {
 
@@ -46,7 +47,12 @@ enum EngineType : uint32_t {
 };
 
 constexpr int kEThreads = 256;
-constexpr int kEMinBlocks = 2;
+// Four blocks per SM (64 registers, some spilled): 512 searches in 78 ms
+// against 87 ms with three blocks of 80 and 109 ms with two of 128.
+constexpr int kEMinBlocks = 4;
+// Pancake sizes whose top-down levels run in windows of 8! states
+// (pancake_window): 10 and more, 90 windows an instance.
+constexpr int kEPancakeWindowsMin = 10;
 constexpr uint32_t kEWindowBitsMax = 16;
 
 struct EngineSlot {
@@ -55,7 +61,8 @@ struct EngineSlot {
     uint32_t type;      // EngineType
     uint32_t state;     // 0 free, 1 active, 2 done (waiting for the host to collect)
     uint32_t depth;     // counts recorded so far
-    uint32_t windows;   // windows of this instance
+    uint32_t windows;   // windows of this instance (flags, bottom-up levels)
+    uint32_t td_windows;  // windows of a top-down level: 8! states each for 10 to 12 pancakes, else the same
     uint32_t bu;        // this level runs bottom-up
     uint32_t can_bu;    // the puzzle allows bottom-up levels (not Hanoi with symmetry)
     uint64_t seen;      // states at depths below the current frontier's
@@ -86,7 +93,10 @@ __global__ void __launch_bounds__(1024) engine_build_queue(EngineDev d) {
     for (uint32_t base = 0; base < d.n_slots; base += 1024) {
         const uint32_t s = base + threadIdx.x;
         uint32_t w = 0;
-        if (s < d.n_slots && d.slots[s].state == 1) { w = d.slots[s].windows; active++; }
+        if (s < d.n_slots && d.slots[s].state == 1) {
+            w = d.slots[s].bu ? d.slots[s].windows : d.slots[s].td_windows;
+            active++;
+        }
         uint32_t incl = w;
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         for (int o = 1; o < 32; o <<= 1) {
@@ -131,9 +141,9 @@ __device__ __forceinline__ void engine_window(const LevelArgs& a, uint64_t windo
     if constexpr (T == kE_P7) level_window<PancakeK<7>, kTwoBit, kEThreads>(a, window, smem, sh);
     if constexpr (T == kE_P8) level_window<PancakeK<8>, kTwoBit, kEThreads>(a, window, smem, sh);
     if constexpr (T == kE_P9) level_window<PancakeK<9>, kTwoBit, kEThreads>(a, window, smem, sh);
-    if constexpr (T == kE_P10) level_window<PancakeK<10>, kTwoBit, kEThreads>(a, window, smem, sh);
-    if constexpr (T == kE_P11) level_window<PancakeK<11>, kTwoBit, kEThreads>(a, window, smem, sh);
-    if constexpr (T == kE_P12) level_window<PancakeK<12>, kTwoBit, kEThreads>(a, window, smem, sh);
+    if constexpr (T == kE_P10) pancake_window<10, kTwoBit, kEThreads>(a, window, smem, sh);
+    if constexpr (T == kE_P11) pancake_window<11, kTwoBit, kEThreads>(a, window, smem, sh);
+    if constexpr (T == kE_P12) pancake_window<12, kTwoBit, kEThreads>(a, window, smem, sh);
     if constexpr (T == kE_H) {
         if (!hanoi_words_ok(a.pz)) {
             level_window<HanoiK, kTwoBit, kEThreads>(a, window, smem, sh);
@@ -298,6 +308,16 @@ __global__ void engine_collect(EngineDev d, uint32_t first, uint32_t n, unsigned
         row[2 + k] = d.counts[uint64_t(s) * d.max_depths + k];
 }
 
+// Admits one search: its slot, cleared counters, the start state's code (CUR
+// = 2: bit 2i, given as a word of the cleared array) and window flag.
+__global__ void engine_admit(EngineDev d, EngineSlot slot, uint32_t s, uint64_t code_word, uint64_t code,
+                             uint64_t flag_window) {
+    slot.args.front[code_word] = code;
+    slot.flags[0][flag_window] = 1;
+    for (int i = 0; i < 8; ++i) d.stats[8ull * s + i] = 0;
+    d.slots[s] = slot;
+}
+
 // Frees the slots the host has collected.
 __global__ void engine_release(EngineDev d, const uint32_t* slots, uint32_t n) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -313,7 +333,6 @@ struct psb_engine {
     uint64_t pool_words = 0;
     uint64_t* pool = nullptr;
     psb::EngineDev d{};
-    std::vector<psb::EngineSlot> host_slots;
     std::vector<uint64_t> slot_off, slot_words, slot_tag;
     std::vector<uint32_t> free_slots;
     std::map<uint64_t, uint64_t> free_space;  // offset -> words (first fit)
@@ -486,7 +505,6 @@ int psb_engine_create(const psb_engine_opts* opts, psb_engine** out) {
     EN_CUDA(cudaMallocHost(&e->h_err, 8));
     EN_CUDA(cudaMalloc(&e->d_staging, 8ull * e->n_slots * (e->max_depths + 2)));
     e->h_staging.resize(size_t(e->n_slots) * (e->max_depths + 2));
-    e->host_slots.assign(e->n_slots, psb::EngineSlot{});
     e->slot_off.assign(e->n_slots, 0);
     e->slot_words.assign(e->n_slots, 0);
     e->slot_tag.assign(e->n_slots, 0);
@@ -555,6 +573,8 @@ int psb_engine_add(psb_engine* e, int kind, int a, int b, uint64_t initial, uint
     slot.state = 1;
     slot.depth = 0;
     slot.windows = windows;
+    slot.td_windows = kind == PSB_PANCAKE && a >= psb::kEPancakeWindowsMin
+                          ? uint32_t(p->n_states / psb::kPancakeWindow) : windows;
     slot.flags[0] = reinterpret_cast<uint8_t*>(e->pool + off + code_words);
     slot.flags[1] = slot.flags[0] + flag_words * 4;
     psb::LevelArgs& la = slot.args;
@@ -573,18 +593,13 @@ int psb_engine_add(psb_engine* e, int kind, int a, int b, uint64_t initial, uint
     // Level 0 sweeps only the start state's window and records flags for level 1.
     la.wflag_cur = slot.flags[0];
     la.wflag_next = slot.flags[1];
+    // In stream order before the next step; four small copies and a wait
+    // here took 20 us a search.
     cudaStream_t st = e->stream;
     EN_CUDA(cudaMemsetAsync(e->pool + off, 0, words * 8, st));
-    static thread_local uint8_t one;
-    one = 1;
-    EN_CUDA(cudaMemcpyAsync(slot.flags[0] + (initial >> wb), &one, 1, cudaMemcpyHostToDevice, st));
-    static thread_local uint64_t word;
-    word = uint64_t(1) << ((2 * initial) & 63);  // code CUR = 2 at the initial state: bit 2i
-    EN_CUDA(cudaMemcpyAsync(e->pool + off + (2 * initial) / 64, &word, 8, cudaMemcpyHostToDevice, st));
-    EN_CUDA(cudaMemsetAsync(e->d.stats + 8ull * s, 0, 64, st));
-    e->host_slots[s] = slot;
-    EN_CUDA(cudaMemcpyAsync(e->d.slots + s, &e->host_slots[s], sizeof(psb::EngineSlot), cudaMemcpyHostToDevice, st));
-    EN_CUDA(cudaStreamSynchronize(st));
+    psb::engine_admit<<<1, 1, 0, st>>>(e->d, slot, s, (2 * initial) / 64, uint64_t(1) << ((2 * initial) & 63),
+                                       initial >> wb);
+    EN_CUDA(cudaGetLastError());
     e->active++;
     *slot_out = s;
     return PSB_OK;
