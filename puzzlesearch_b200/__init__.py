@@ -741,16 +741,17 @@ def frontier_encode(d_bits, first_bit, n_bits, d_out=None, out_cap=0, stream=Non
     (stream_bytes, block_table, n_blocks); with d_out=None only sizes it."""
     nbytes = ctypes.c_uint64()
     nb = ctypes.c_uint32()
+    # as many blocks as the range can hold (262,144 offsets each)
+    rows = 0 if d_out is None else max(1, (n_bits + 262143) // 262144)
+    blocks = (CodecBlock * rows)() if rows else None
     rc = lib().psb_frontier_encode(ctypes.cast(d_bits, u64p), first_bit, n_bits, d_out, out_cap,
-                                   ctypes.byref(nbytes), None, 0, ctypes.byref(nb), stream)
+                                   ctypes.byref(nbytes), blocks, rows, ctypes.byref(nb), stream)
     if d_out is None:
         if rc not in (0, -4):
             _check(rc)
         return nbytes.value, None, nb.value
-    blocks = (CodecBlock * max(nb.value, 1))()
-    _check(lib().psb_frontier_encode(ctypes.cast(d_bits, u64p), first_bit, n_bits, d_out, out_cap,
-                                     ctypes.byref(nbytes), blocks, nb.value, ctypes.byref(nb), stream))
-    return nbytes.value, blocks, nb.value
+    _check(rc)
+    return nbytes.value, (CodecBlock * max(nb.value, 1)).from_buffer(blocks), nb.value
 
 
 def frontier_decode(d_stream, blocks, n_blocks, d_bits, first_bit, n_bits, stream=None):

@@ -114,42 +114,6 @@ __global__ void __launch_bounds__(kScanT) k_scan_small(unsigned long long* v, ui
     if (threadIdx.x == 0) *total = carry;
 }
 
-// Large exclusive scan in place: group sums (4096 values per block), a scan of
-// the group sums, then a per-group pass.
-__global__ void k_group_sums(const unsigned long long* v, uint64_t n, unsigned long long* gsum) {
-    const uint64_t base = uint64_t(blockIdx.x) * kT * 16 + uint64_t(threadIdx.x) * 16;
-    unsigned long long c = 0;
-    for (int k = 0; k < 16; ++k) if (base + k < n) c += v[base + k];
-    __shared__ unsigned long long s[kT];
-    s[threadIdx.x] = c;
-    __syncthreads();
-    for (int o = kT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) gsum[blockIdx.x] = s[0];
-}
-
-__global__ void k_group_scan(unsigned long long* v, uint64_t n, const unsigned long long* gsum) {
-    const uint64_t base = uint64_t(blockIdx.x) * kT * 16 + uint64_t(threadIdx.x) * 16;
-    unsigned long long x[16], c = 0;
-    for (int k = 0; k < 16; ++k) { x[k] = base + k < n ? v[base + k] : 0; c += x[k]; }
-    __shared__ unsigned long long s[kT];
-    s[threadIdx.x] = c;
-    __syncthreads();
-    for (int o = 1; o < kT; o <<= 1) {
-        const unsigned long long y = threadIdx.x >= o ? s[threadIdx.x - o] : 0;
-        __syncthreads();
-        s[threadIdx.x] += y;
-        __syncthreads();
-    }
-    unsigned long long run = gsum[blockIdx.x] + s[threadIdx.x] - c;
-    for (int k = 0; k < 16; ++k) {
-        if (base + k < n) v[base + k] = run;
-        run += x[k];
-    }
-}
-
 // Inclusive block-wide sum scan of one value per thread (kT threads).
 __device__ __forceinline__ uint32_t block_inclusive_scan(uint32_t v, uint32_t* warp_tot) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -181,20 +145,26 @@ __device__ __forceinline__ void chunk_total(uint32_t c, unsigned long long* out)
 
 __device__ __forceinline__ uint32_t vbytes(uint32_t x) { return x >> 24 ? 4 : x >> 16 ? 3 : x >> 8 ? 2 : 1; }
 
+// A block of up to kBlock offsets.
 struct BlockInfo {
-    unsigned long long out_off;  // byte offset of the block in the stream
-    uint32_t count, first, last, is_bitmap;
+    unsigned long long out_off;  // byte offset of the block in the segment's stream
     unsigned long long bytes;
+    uint32_t count, first, last, is_bitmap;
+    uint32_t svi, pad;  // StreamVInt blocks: which one (its place in the offset list)
 };
 
-// A StreamVInt block in tuple order: its first tuple and its block number.
-struct SviRef {
-    unsigned long long tuple0;
-    uint32_t block, pad;
-};
+// One segment's result, on the device (EncTotals) and read by the host.
+using psb::EncTotals;
+
+// StreamVInt blocks are worked on in parts of kPartTuples tuples.
+constexpr uint32_t kPartTuples = 4096, kParts = kBlock / 4 / kPartTuples;
+// Bitmap blocks in parts of kPartWords words: a bitmap block's bitmap is
+// smaller than 10 bits per offset, so 40 parts hold any.
+constexpr uint32_t kPartWords = 1024, kBitmapParts = 40;
+static_assert(uint64_t(kBitmapParts) * kPartWords * 64 >= uint64_t(kBlock) * 10, "every bitmap block's words have a part");
 
 // Writes the ascending offsets of the set bits that fall in StreamVInt
-// blocks, at their rank (offset list position = rank; bitmap blocks need no
+// blocks into their block's place of the offset list (bitmap blocks need no
 // list: their words are copied from the bitmap).  One CTA per chunk of
 // kT * 16 words; warp w takes the chunk's words 512 w .. 512 w + 511, 32 at a
 // time, lane l word 32 i + l, so every load is coalesced.  A first pass
@@ -203,13 +173,14 @@ struct SviRef {
 // each lane's offsets by a warp scan, so neighbouring lanes store
 // neighbouring ranks.
 __global__ void __launch_bounds__(kT) k_compact(const uint64_t* bits, uint64_t n_words, uint64_t n_bits,
-                                                const unsigned long long* bsum, uint64_t nbs, uint64_t count,
-                                                const BlockInfo* blocks, uint32_t* idx) {
+                                                const unsigned long long* bsum, uint64_t nbs, const EncTotals* totals,
+                                                const BlockInfo* blocks, uint32_t cap_refs, uint32_t* idx) {
     __shared__ uint32_t warp_tot[kT / 32];
+    if (totals->n_refs == 0 || totals->n_refs > cap_refs) return;
     // Chunks with no offsets, or whose offsets all fall in bitmap blocks,
     // have nothing to list (uniform over the CTA: the chunk's rank range).
     const unsigned long long r_lo = bsum[blockIdx.x];
-    const unsigned long long r_hi = blockIdx.x + 1 < nbs ? bsum[blockIdx.x + 1] : count;
+    const unsigned long long r_hi = blockIdx.x + 1 < nbs ? bsum[blockIdx.x + 1] : totals->count;
     if (r_hi == r_lo) return;
     bool all_bitmap = true;
     for (uint64_t b = r_lo / kBlock; b <= (r_hi - 1) / kBlock; ++b) all_bitmap = all_bitmap && blocks[b].is_bitmap;
@@ -255,8 +226,10 @@ __global__ void __launch_bounds__(kT) k_compact(const uint64_t* bits, uint64_t n
             const uint64_t word = __shfl_sync(0xFFFFFFFFu, m, int(lo));
             if (k < total) {
                 const unsigned long long rank = r + k;
-                if (!blocks[rank / kBlock].is_bitmap)
-                    idx[rank] = uint32_t((w0 + 32u * i - lane + lo) * 64 + psb::select_bit(word, k - before));
+                const BlockInfo& b = blocks[rank / kBlock];
+                if (!b.is_bitmap)
+                    idx[uint64_t(b.svi) * kBlock + rank % kBlock] =
+                        uint32_t((w0 + 32u * i - lane + lo) * 64 + psb::select_bit(word, k - before));
             }
         }
         r += total;
@@ -266,160 +239,286 @@ __global__ void __launch_bounds__(kT) k_compact(const uint64_t* bits, uint64_t n
 // First and last offset of every block (ranks b * kBlock and the block's
 // last rank), by select: the chunk holding the rank from the chunk prefix
 // sums (bsum, chunks of kT * 16 words), then a block scan of that chunk's
-// per-thread counts (thread t: words 16 t .. 16 t + 15).  CTAs 2b and 2b + 1
+// per-thread counts (thread t: words 16 t .. 16 t + 15).  Items 2b and 2b + 1
 // serve block b.
 __global__ void __launch_bounds__(kT) k_select_blocks(const uint64_t* bits, uint64_t n_words, uint64_t n_bits,
-                                                      const unsigned long long* bsum, uint64_t nbs, uint64_t count,
-                                                      BlockInfo* blocks, uint32_t nb) {
+                                                      const unsigned long long* bsum, uint64_t nbs,
+                                                      const EncTotals* totals, BlockInfo* blocks) {
     __shared__ uint32_t warp_tot[kT / 32];
-    const uint32_t b = blockIdx.x / 2;
-    const bool last = blockIdx.x & 1;
-    const uint64_t end = (uint64_t(b) + 1) * kBlock < count ? (uint64_t(b) + 1) * kBlock : count;
-    const uint64_t r = last ? end - 1 : uint64_t(b) * kBlock;
-    uint64_t lo = 0, hi = nbs;  // largest chunk lo with bsum[lo] <= r (bsum[0] = 0)
-    while (hi - lo > 1) {
-        const uint64_t mid = (lo + hi) / 2;
-        if (bsum[mid] <= r) lo = mid; else hi = mid;
-    }
-    const uint64_t rem = r - bsum[lo];
-    const uint64_t w0 = lo * kT * 16 + uint64_t(threadIdx.x) * 16;
-    uint64_t v[16];
-    uint32_t c = 0;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-        v[k] = w0 + k < n_words ? masked_word(bits, w0 + k, n_words, n_bits) : 0;
-        c += __popcll(v[k]);
-    }
-    const uint32_t inc = block_inclusive_scan(c, warp_tot);
-    const uint32_t exc = inc - c;
-    if (rem < exc || rem >= inc) return;  // exactly one thread holds the rank
-    uint64_t left = rem - exc;
-    for (int k = 0; k < 16; ++k) {
-        const uint32_t ck = __popcll(v[k]);
-        if (left < ck) {
-            uint64_t x = v[k];
-            for (uint64_t i = 0; i < left; ++i) x &= x - 1;
-            const uint32_t pos = uint32_t((w0 + k) * 64 + (__ffsll((long long)x) - 1));
-            if (last) blocks[b].last = pos; else blocks[b].first = pos;
-            return;
+    const uint64_t count = totals->count, nb = (count + kBlock - 1) / kBlock;
+    for (uint64_t item = blockIdx.x; item < 2 * nb; item += gridDim.x) {
+        const uint64_t b = item / 2;
+        const bool last = item & 1;
+        const uint64_t end = (b + 1) * kBlock < count ? (b + 1) * kBlock : count;
+        const uint64_t r = last ? end - 1 : b * kBlock;
+        uint64_t lo = 0, hi = nbs;  // largest chunk lo with bsum[lo] <= r (bsum[0] = 0)
+        while (hi - lo > 1) {
+            const uint64_t mid = (lo + hi) / 2;
+            if (bsum[mid] <= r) lo = mid; else hi = mid;
         }
-        left -= ck;
+        const uint64_t rem = r - bsum[lo];
+        const uint64_t w0 = lo * kT * 16 + uint64_t(threadIdx.x) * 16;
+        uint64_t v[16];
+        uint32_t c = 0;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            v[k] = w0 + k < n_words ? masked_word(bits, w0 + k, n_words, n_bits) : 0;
+            c += __popcll(v[k]);
+        }
+        const uint32_t inc = block_inclusive_scan(c, warp_tot);  // ends with a barrier
+        const uint32_t exc = inc - c;
+        if (rem < exc || rem >= inc) continue;  // exactly one thread holds the rank
+        uint32_t left = uint32_t(rem - exc);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const uint32_t ck = __popcll(v[k]);
+            if (left < ck) {
+                const uint32_t pos = uint32_t((w0 + k) * 64 + psb::select_bit(v[k], left));
+                if (last) blocks[b].last = pos; else blocks[b].first = pos;
+                left = 0xFFFFFFFFu;  // found
+            } else if (left != 0xFFFFFFFFu) {
+                left -= ck;
+            }
+        }
     }
+}
+
+// Inclusive scan of one value per thread over a CTA of kScanT threads.
+__device__ __forceinline__ unsigned long long scan_cta(unsigned long long v, unsigned long long* warp_tot,
+                                                       unsigned long long* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += y;
+    }
+    if (lane == 31) warp_tot[warp] = v;
+    __syncthreads();
+    unsigned long long before = 0, all = 0;
+    for (int w = 0; w < kScanT / 32; ++w) {
+        if (w < warp) before += warp_tot[w];
+        all += warp_tot[w];
+    }
+    __syncthreads();
+    *total = all;
+    return before + v;
 }
 
 // FrontierCompression::Encode (FrontierCompression.cpp:92-102): a block is a
 // bitmap block when it holds more than 128 offsets and its bitmap is smaller
-// than 10 bits per offset.
-// With operator bits (force_svi) every block is a StreamVInt block, as
-// CompressedFrontierWriter writes them (Common/CompressedFrontier.cpp:63-70).
-__global__ void k_block_decide(uint64_t count, BlockInfo* blocks, uint32_t nb, int force_svi) {
-    const uint32_t b = blockIdx.x * kT + threadIdx.x;
-    if (b >= nb) return;
-    BlockInfo& bi = blocks[b];
-    const uint64_t r0 = uint64_t(b) * kBlock;
-    const uint32_t n = uint32_t(count - r0 < kBlock ? count - r0 : kBlock);
-    bi.count = n;
-    const uint64_t bm_bytes = (uint64_t(bi.last) - bi.first + 63) / 64 * 8 + 8;
-    bi.is_bitmap = (!force_svi && n > 128 && bm_bytes * 8 < uint64_t(n) * 10 - 8) ? 1 : 0;
-    bi.bytes = bi.is_bitmap ? bm_bytes : 0;
-    bi.out_off = 0;
-}
-
-// Value of rank position k (0-based) of block b after the in-place delta, 0 past the count.
-__device__ __forceinline__ uint32_t delta_at(const uint32_t* idx, uint64_t r0, uint32_t count, uint32_t k) {
-    if (k >= count) return 0;
-    const uint32_t v = idx[r0 + k];
-    return k == 0 ? v : v - idx[r0 + k - 1];
-}
-
-// The StreamVInt block that holds tuple t (the last ref with tuple0 <= t).
-__device__ __forceinline__ uint32_t svi_of(const SviRef* refs, uint32_t n_refs, uint64_t t) {
-    uint32_t lo = 0, hi = n_refs;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (refs[mid].tuple0 <= t) lo = mid; else hi = mid;
+// than 10 bits per offset.  With operator bits (force_svi) every block is a
+// StreamVInt block, as CompressedFrontierWriter writes them
+// (Common/CompressedFrontier.cpp:63-70).  One CTA; the StreamVInt blocks are
+// numbered in order.
+__global__ void __launch_bounds__(kScanT) k_decide(EncTotals* totals, BlockInfo* blocks, uint32_t* refs,
+                                                   int force_svi) {
+    __shared__ unsigned long long warp_tot[kScanT / 32];
+    const uint64_t count = totals->count, nb = (count + kBlock - 1) / kBlock;
+    unsigned long long n_refs = 0;
+    for (uint64_t b0 = 0; b0 < nb; b0 += kScanT) {
+        const uint64_t b = b0 + threadIdx.x;
+        uint32_t svi = 0;
+        if (b < nb) {
+            BlockInfo& bi = blocks[b];
+            const uint64_t r0 = b * kBlock;
+            const uint32_t n = uint32_t(count - r0 < kBlock ? count - r0 : kBlock);
+            bi.count = n;
+            const uint64_t bm_bytes = (uint64_t(bi.last) - bi.first + 63) / 64 * 8 + 8;
+            bi.is_bitmap = (!force_svi && n > 128 && bm_bytes * 8 < uint64_t(n) * 10 - 8) ? 1 : 0;
+            bi.bytes = bm_bytes;  // of a bitmap block; k_layout fills in the others
+            svi = !bi.is_bitmap;
+        }
+        unsigned long long total;
+        const unsigned long long at = n_refs + scan_cta(svi, warp_tot, &total) - svi;
+        if (svi) {
+            blocks[b].svi = uint32_t(at);
+            refs[at] = uint32_t(b);
+        }
+        n_refs += total;
     }
-    return lo;
+    if (threadIdx.x == 0) {
+        totals->nb = uint32_t(nb);
+        totals->n_refs = uint32_t(n_refs);
+    }
 }
 
-// Tuple lengths of the StreamVInt blocks: 1 descriptor byte + 1..4 bytes per value.
-__global__ void k_tuple_len(const uint32_t* idx, const BlockInfo* blocks, const SviRef* refs, uint32_t n_refs,
-                            uint64_t tuples, unsigned long long* tlen) {
-    const uint64_t t = blockIdx.x * uint64_t(kT) + threadIdx.x;
-    if (t >= tuples) return;
-    const SviRef ref = refs[svi_of(refs, n_refs, t)];
-    const uint32_t k = uint32_t(t - ref.tuple0) * 4;
-    const uint32_t count = blocks[ref.block].count;
-    const uint64_t r0 = uint64_t(ref.block) * kBlock;
-    uint32_t len = 1;
-    for (int q = 0; q < 4; ++q) len += vbytes(delta_at(idx, r0, count, k + q));
-    tlen[t] = len;
+// The four deltas of tuple t of a block (0 past its count; the first value
+// of a block is itself) and the tuple's length: 1 descriptor byte and 1..4
+// bytes per value.
+__device__ __forceinline__ uint32_t tuple_of(const uint32_t* v, uint32_t count, uint32_t t, uint32_t (&x)[4]) {
+    const uint32_t k = 4 * t;
+    const uint4 q = *reinterpret_cast<const uint4*>(v + k);
+    const uint32_t prev = k ? v[k - 1] : 0;
+    x[0] = k < count ? q.x - prev : 0;
+    x[1] = k + 1 < count ? q.y - q.x : 0;
+    x[2] = k + 2 < count ? q.z - q.y : 0;
+    x[3] = k + 3 < count ? q.w - q.z : 0;
+    return 1 + vbytes(x[0]) + vbytes(x[1]) + vbytes(x[2]) + vbytes(x[3]);
 }
 
-// Bytes of each StreamVInt block: header, tuples and, with operator bits,
-// the bounds (one nibble per padded value, StreamVInt.cpp:253-275).
-__global__ void k_block_bytes(BlockInfo* blocks, const SviRef* refs, uint32_t n_refs,
-                              const unsigned long long* tscan, uint64_t tuples, unsigned long long total,
-                              int with_ops) {
-    const uint32_t j = blockIdx.x * kT + threadIdx.x;
-    if (j >= n_refs) return;
-    BlockInfo& bi = blocks[refs[j].block];
-    const uint64_t t0 = refs[j].tuple0, t1 = j + 1 < n_refs ? refs[j + 1].tuple0 : tuples;
-    const unsigned long long end = t1 < tuples ? tscan[t1] : total;
-    bi.bytes = 4 + (end - tscan[t0]) + (with_ops ? (uint64_t(bi.count) + 7) / 8 * 4 : 0);
+__device__ __forceinline__ uint32_t tuples_of(uint32_t count) { return uint32_t((uint64_t(count) + 7) / 8 * 2); }
+
+// psum[ref * kParts + p] = bytes of the tuples of part p of StreamVInt block `ref`.
+__global__ void __launch_bounds__(kT) k_part_bytes(const uint32_t* idx, const EncTotals* totals,
+                                                   const BlockInfo* blocks, const uint32_t* refs, uint32_t cap_refs,
+                                                   unsigned long long* psum) {
+    if (totals->n_refs > cap_refs) return;
+    const uint32_t items = totals->n_refs * kParts;
+    for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const uint32_t ref = item / kParts, count = blocks[refs[ref]].count, tuples = tuples_of(count);
+        const uint32_t t0 = (item % kParts) * kPartTuples;
+        uint32_t c = 0;
+        for (uint32_t t = t0 + threadIdx.x; t < t0 + kPartTuples && t < tuples; t += kT) {
+            uint32_t x[4];
+            c += tuple_of(idx + uint64_t(ref) * kBlock, count, t, x);
+        }
+        chunk_total(c, psum + item);
+        __syncthreads();
+    }
+}
+
+// Places the blocks: each StreamVInt block's bytes (header, tuples and, with
+// operator bits, one nibble per padded value, StreamVInt.cpp:253-275), its
+// parts' first bytes (psum becomes their exclusive prefix), each block's
+// offset in the stream and the segment's place: at `first_off`, or after the
+// segment before it.  One CTA.
+__global__ void __launch_bounds__(kScanT) k_layout(EncTotals* totals, BlockInfo* blocks, unsigned long long* psum,
+                                                   uint32_t cap_refs, int with_ops, int first,
+                                                   unsigned long long first_off) {
+    __shared__ unsigned long long warp_tot[kScanT / 32];
+    const uint64_t nb = totals->nb;
+    const bool listed = totals->n_refs <= cap_refs;
+    unsigned long long off = 0;
+    for (uint64_t b0 = 0; b0 < nb; b0 += kScanT) {
+        const uint64_t b = b0 + threadIdx.x;
+        unsigned long long bytes = 0;
+        if (b < nb) {
+            BlockInfo& bi = blocks[b];
+            if (!bi.is_bitmap) {
+                unsigned long long t = 0;
+                if (listed) {
+                    for (uint32_t p = 0; p < kParts; ++p) {
+                        const unsigned long long own = psum[uint64_t(bi.svi) * kParts + p];
+                        psum[uint64_t(bi.svi) * kParts + p] = t;
+                        t += own;
+                    }
+                }
+                bi.bytes = 4 + t + (with_ops ? (uint64_t(bi.count) + 7) / 8 * 4 : 0);
+            }
+            bytes = bi.bytes;
+        }
+        unsigned long long total;
+        const unsigned long long incl = scan_cta(bytes, warp_tot, &total);
+        if (b < nb) blocks[b].out_off = off + incl - bytes;
+        off += total;
+    }
+    if (threadIdx.x == 0) {
+        totals->bytes = off;
+        totals->off = first ? first_off : totals[-1].off + totals[-1].bytes;
+    }
+}
+
+// The segment's stream, or NULL when it was not planned whole or does not fit.
+__device__ __forceinline__ uint8_t* stream_place(const EncTotals* totals, uint32_t cap_refs, uint8_t* out,
+                                                 unsigned long long out_cap) {
+    if (totals->n_refs > cap_refs || totals->off + totals->bytes > out_cap) return nullptr;
+    return out + totals->off;
+}
+
+// The CTA's threads write n bytes of shared memory (from a 4-byte boundary,
+// readable 4 bytes past n) to dst (any alignment): whole aligned words, and
+// the few bytes at the ends.
+__device__ __forceinline__ void store_bytes(uint8_t* dst, const uint32_t* src, uint32_t n) {
+    const uint8_t* sb = reinterpret_cast<const uint8_t*>(src);
+    const uint32_t to_word = uint32_t(0 - reinterpret_cast<uintptr_t>(dst)) & 3u;
+    const uint32_t head = to_word < n ? to_word : n, words = (n - head) / 4, tail = head + 4 * words;
+    if (threadIdx.x < head) dst[threadIdx.x] = sb[threadIdx.x];
+    for (uint32_t j = threadIdx.x; j < words; j += kT)
+        *reinterpret_cast<uint32_t*>(dst + head + 4 * j) = __funnelshift_r(src[j], src[j + 1], 8 * head);
+    if (threadIdx.x < n - tail) dst[tail + threadIdx.x] = sb[tail + threadIdx.x];
+}
+
+// The tuples of the StreamVInt blocks, part by part, kT tuples at a time
+// through shared memory, so that the stores are whole words.
+__global__ void __launch_bounds__(kT) k_write_svi(const uint32_t* idx, const EncTotals* totals,
+                                                  const BlockInfo* blocks, const uint32_t* refs, uint32_t cap_refs,
+                                                  const unsigned long long* psum, uint8_t* out,
+                                                  unsigned long long out_cap) {
+    __shared__ uint32_t buf[kT * 17 / 4 + 2];
+    __shared__ uint32_t warp_tot[kT / 32], round_bytes;
+    uint8_t* place = stream_place(totals, cap_refs, out, out_cap);
+    if (!place) return;
+    uint8_t* sb = reinterpret_cast<uint8_t*>(buf);
+    const uint32_t items = totals->n_refs * kParts;
+    for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const uint32_t ref = item / kParts, part = item % kParts;
+        const BlockInfo bi = blocks[refs[ref]];
+        const uint32_t tuples = tuples_of(bi.count), t0 = part * kPartTuples;
+        if (t0 >= tuples) continue;
+        uint8_t* p = place + bi.out_off;
+        if (part == 0 && threadIdx.x < 4) p[threadIdx.x] = uint8_t(bi.count >> (8 * threadIdx.x));
+        p += 4 + psum[item];
+        for (uint32_t r = t0; r < t0 + kPartTuples && r < tuples; r += kT) {
+            const uint32_t t = r + threadIdx.x;
+            uint32_t x[4], len = 0;
+            if (t < tuples) len = tuple_of(idx + uint64_t(ref) * kBlock, bi.count, t, x);
+            const uint32_t incl = block_inclusive_scan(len, warp_tot);
+            if (threadIdx.x == kT - 1) round_bytes = incl;
+            if (len) {
+                uint32_t at = incl - len, desc = 0, pos = at + 1;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint32_t nbytes = vbytes(x[q]);
+                    desc |= (nbytes - 1) << (2 * q);
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; ++i)
+                        if (i < nbytes) sb[pos + i] = uint8_t(x[q] >> (8 * i));
+                    pos += nbytes;
+                }
+                sb[at] = uint8_t(desc);
+            }
+            __syncthreads();
+            const uint32_t n = round_bytes;
+            store_bytes(p, buf, n);
+            p += n;
+            __syncthreads();
+        }
+    }
 }
 
 // Bounds of the StreamVInt blocks (StreamVInt::EncodeBounds,
 // StreamVInt.cpp:139-147,193-198): the operator nibble of each value, 8 per
 // group packed as bytes b_q | b_(q+4) << 4, after the block's tuples.  The
 // nibble of offset v is state nib_first + v of the 4-bit array `nib` (NULL:
-// every nibble is 0); values past the count have nibble 0.  One thread per
-// group of 8 values (two tuples).
-__global__ void k_write_bounds(const uint32_t* idx, const BlockInfo* blocks, const SviRef* refs, uint32_t n_refs,
-                               uint64_t groups, const uint64_t* nib, uint64_t nib_first, uint8_t* out) {
-    const uint64_t g = blockIdx.x * uint64_t(kT) + threadIdx.x;
-    if (g >= groups) return;
-    const SviRef ref = refs[svi_of(refs, n_refs, 2 * g)];
-    const uint32_t k = uint32_t(2 * g - ref.tuple0) * 4;  // first value of the group in its block
-    const BlockInfo bi = blocks[ref.block];
-    const uint64_t r0 = uint64_t(ref.block) * kBlock;
-    const uint64_t adj = (uint64_t(bi.count) + 7) / 8 * 8;
-    uint8_t* p = out + bi.out_off + bi.bytes - adj / 2 + k / 2;
-    uint32_t b[8];
+// every nibble is 0); values past the count have nibble 0.
+__global__ void __launch_bounds__(kT) k_write_bounds(const uint32_t* idx, const EncTotals* totals,
+                                                     const BlockInfo* blocks, const uint32_t* refs, uint32_t cap_refs,
+                                                     const uint64_t* nib, uint64_t nib_first, uint8_t* out,
+                                                     unsigned long long out_cap) {
+    uint8_t* place = stream_place(totals, cap_refs, out, out_cap);
+    if (!place) return;
+    const uint32_t items = totals->n_refs * kParts;
+    for (uint32_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const uint32_t ref = item / kParts, part = item % kParts;
+        const BlockInfo bi = blocks[refs[ref]];
+        const uint32_t groups = tuples_of(bi.count) / 2, g0 = part * (kPartTuples / 2);
+        const uint32_t* v = idx + uint64_t(ref) * kBlock;
+        uint8_t* bounds = place + bi.out_off + bi.bytes - uint64_t(groups) * 4;
+        for (uint32_t g = g0 + threadIdx.x; g < g0 + kPartTuples / 2 && g < groups; g += kT) {
+            uint32_t b[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        b[j] = 0;
-        if (nib && k + j < bi.count) {
-            const uint64_t state = nib_first + idx[r0 + k + j];
-            b[j] = uint32_t(nib[state >> 4] >> (4 * (state & 15))) & 15u;
+            for (int j = 0; j < 8; ++j) {
+                b[j] = 0;
+                if (nib && 8 * g + j < bi.count) {
+                    const uint64_t state = nib_first + v[8 * g + j];
+                    b[j] = uint32_t(nib[state >> 4] >> (4 * (state & 15))) & 15u;
+                }
+            }
+            uint8_t* p = bounds + 4ull * g;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) p[q] = uint8_t(b[q] | (b[q + 4] << 4));
         }
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) p[q] = uint8_t(b[q] | (b[q + 4] << 4));
-}
-
-__global__ void k_write_svi(const uint32_t* idx, const BlockInfo* blocks, const SviRef* refs, uint32_t n_refs,
-                            uint64_t tuples, const unsigned long long* tscan, uint8_t* out) {
-    const uint64_t t = blockIdx.x * uint64_t(kT) + threadIdx.x;
-    if (t >= tuples) return;
-    const SviRef ref = refs[svi_of(refs, n_refs, t)];
-    const uint32_t k = uint32_t(t - ref.tuple0) * 4;
-    const BlockInfo bi = blocks[ref.block];
-    const uint64_t r0 = uint64_t(ref.block) * kBlock;
-    uint8_t* p = out + bi.out_off + 4 + (tscan[t] - tscan[ref.tuple0]);
-    if (k == 0) {
-        uint8_t* h = out + bi.out_off;
-        h[0] = uint8_t(bi.count); h[1] = uint8_t(bi.count >> 8); h[2] = uint8_t(bi.count >> 16); h[3] = uint8_t(bi.count >> 24);
-    }
-    uint8_t desc = 0;
-    int pos = 1;
-    for (int q = 0; q < 4; ++q) {
-        const uint32_t x = delta_at(idx, r0, bi.count, k + q);
-        const uint32_t nbytes = vbytes(x);
-        desc |= uint8_t((nbytes - 1) << (2 * q));
-        for (uint32_t i = 0; i < nbytes; ++i) p[pos++] = uint8_t(x >> (8 * i));
-    }
-    p[0] = desc;
 }
 
 // Bitmap block: bit j of output word i is state first + 1 + 64 i + j (<= last).
@@ -436,66 +535,63 @@ __device__ __forceinline__ uint64_t live_word(const uint64_t* bits, uint64_t w, 
     return chunk_empty(bsum, nbs, count, w) ? 0 : masked_word(bits, w, n_words, n_bits);
 }
 
-__global__ void k_write_bitmap(const uint64_t* bits, uint64_t n_words, uint64_t n_bits, const BlockInfo* blocks,
-                               const unsigned long long* bsum, uint64_t nbs, uint64_t count, uint8_t* out) {
-    const BlockInfo bi = blocks[blockIdx.y];
-    if (!bi.is_bitmap) return;
-    const uint64_t words = (uint64_t(bi.last) - bi.first + 63) / 64;
-    uint8_t* p = out + bi.out_off;
-    const uint64_t i = blockIdx.x * uint64_t(kT) + threadIdx.x;
-    if (i == 0) {
-        const uint32_t h = uint32_t(words) | kMap;
-        for (int q = 0; q < 4; ++q) p[q] = uint8_t(h >> (8 * q));
-        for (int q = 0; q < 4; ++q) p[4 + q] = uint8_t(bi.first >> (8 * q));
+__global__ void __launch_bounds__(kT) k_write_bitmap(const uint64_t* bits, uint64_t n_words, uint64_t n_bits,
+                                                     const EncTotals* totals, const BlockInfo* blocks,
+                                                     const unsigned long long* bsum, uint64_t nbs, uint32_t cap_refs,
+                                                     uint8_t* out, unsigned long long out_cap) {
+    __shared__ uint64_t buf[kPartWords + 1];
+    uint8_t* place = stream_place(totals, cap_refs, out, out_cap);
+    if (!place || totals->n_refs == totals->nb) return;
+    const uint64_t count = totals->count, items = uint64_t(totals->nb) * kBitmapParts;
+    for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const uint32_t part = uint32_t(item % kBitmapParts);
+        const BlockInfo bi = blocks[item / kBitmapParts];
+        const uint32_t words = uint32_t((uint64_t(bi.last) - bi.first + 63) / 64), i0 = part * kPartWords;
+        if (!bi.is_bitmap || (i0 >= words && part)) continue;
+        uint8_t* p = place + bi.out_off;
+        if (part == 0 && threadIdx.x < 8) {
+            const uint64_t h = (words | kMap) | (uint64_t(bi.first) << 32);
+            p[threadIdx.x] = uint8_t(h >> (8 * threadIdx.x));
+        }
+        const uint32_t n = i0 >= words ? 0 : words - i0 < kPartWords ? words - i0 : kPartWords;
+        for (uint32_t i = threadIdx.x; i < n; i += kT) {
+            const uint64_t start = uint64_t(bi.first) + 1 + 64ull * (i0 + i);  // first state of this output word
+            const uint64_t w0 = start >> 6, sh = start & 63;
+            uint64_t v = live_word(bits, w0, n_words, n_bits, bsum, nbs, count) >> sh;
+            if (sh && w0 + 1 < n_words) v |= live_word(bits, w0 + 1, n_words, n_bits, bsum, nbs, count) << (64 - sh);
+            if (start + 63 > bi.last) {  // last state this word covers
+                const uint64_t keep = uint64_t(bi.last) - start + 1;  // 0..63
+                v &= (uint64_t(1) << keep) - 1;
+            }
+            buf[i] = v;
+        }
+        __syncthreads();
+        store_bytes(p + 8 + 8ull * i0, reinterpret_cast<const uint32_t*>(buf), 8 * n);
+        __syncthreads();
     }
-    if (i >= words) return;
-    const uint64_t start = uint64_t(bi.first) + 1 + 64 * i;  // first state of this output word
-    const uint64_t w0 = start >> 6, sh = start & 63;
-    uint64_t v = live_word(bits, w0, n_words, n_bits, bsum, nbs, count) >> sh;
-    if (sh && w0 + 1 < n_words) v |= live_word(bits, w0 + 1, n_words, n_bits, bsum, nbs, count) << (64 - sh);
-    const uint64_t hi = start + 63;  // last state this word covers
-    if (hi > bi.last) {
-        const uint64_t keep = uint64_t(bi.last) - start + 1;  // 0..63
-        v &= keep >= 64 ? ~uint64_t(0) : ((uint64_t(1) << keep) - 1);
-    }
-    for (int q = 0; q < 8; ++q) p[8 + 8 * i + q] = uint8_t(v >> (8 * q));
-}
-
-// Device scratch of the encoder, grown on demand and kept between segments
-// (a search that spills every level's frontier encodes many segments).
-struct Scratch {
-    unsigned long long *bsum = nullptr, *tot = nullptr, *tlen = nullptr, *gsum = nullptr;
-    uint32_t* idx = nullptr;
-    BlockInfo* blocks = nullptr;
-    SviRef* refs = nullptr;
-    size_t cap_bsum = 0, cap_tot = 0, cap_tlen = 0, cap_gsum = 0, cap_idx = 0, cap_blocks = 0, cap_refs = 0;
-};
-
-template <class T>
-int grow(T** p, size_t* cap, size_t need) {
-    if (need <= *cap) return PSB_OK;
-    const size_t want = need + need / 4;
-    CD_CUDA(cudaFree(*p));
-    *p = nullptr;
-    *cap = 0;
-    CD_CUDA(cudaMalloc(reinterpret_cast<void**>(p), want));
-    *cap = want;
-    return PSB_OK;
 }
 
 }  // namespace
 
 namespace psb {
 
+// Encodes segments in stream order without host round trips: every size
+// that depends on the segment (offsets, blocks, tuples, bytes) stays in its
+// EncTotals on the device, and the launches cover whatever it turns out to
+// be.  Only the offset list of the StreamVInt blocks has a capacity
+// (cap_refs blocks); a segment that needs more, or does not fit the output,
+// is planned but not written, and its totals say so.  (With four round
+// trips a segment, 81 depths of 13-disk Hanoi took 16 ms to encode.)
 struct SegmentEncoder {
-    Scratch x;
-    std::vector<BlockInfo> hb;
-    std::vector<SviRef> hrefs;
-    // The planned segment.
-    const uint64_t* bits = nullptr;
-    uint64_t n_bits = 0, n_words = 0, count = 0, tuples = 0, bytes = 0, max_words = 1;
-    uint32_t nb = 0, n_refs = 0;
-    bool any_bitmap = false;
+    uint8_t *fixed = nullptr, *lists = nullptr;  // sized by the segment / by cap_refs
+    size_t cap_fixed = 0;
+    EncTotals* totals = nullptr;
+    uint32_t cap_totals = 0;
+    // parts of the buffers
+    unsigned long long *bsum = nullptr, *psum = nullptr;
+    BlockInfo* blocks = nullptr;
+    uint32_t *refs = nullptr, *idx = nullptr;
+    uint32_t cap_refs = 0;
     uint64_t launches = 0;  // kernels launched since the last encoder_take_launches
     // Operator bits (set_ops): every block StreamVInt with bounds, the nibble
     // of offset v being state ops_first + v of ops_nib (NULL: all zero).
@@ -503,132 +599,124 @@ struct SegmentEncoder {
     const uint64_t* ops_nib = nullptr;
     uint64_t ops_first = 0;
 
-    void set_ops(bool on, const uint64_t* nib, uint64_t first) {
-        with_ops = on;
-        ops_nib = nib;
-        ops_first = first;
+    // The buffers come from the device's pool in stream order; earlier
+    // segments on other streams have been waited for by their callers.
+    template <class T>
+    static int replace(T** p, size_t bytes, cudaStream_t s) {
+        cudaMemPool_t pool = nullptr;
+        if (int rc = scratch_pool(&pool)) return rc;
+        if (*p) CD_CUDA(cudaFreeAsync(*p, s));
+        *p = nullptr;
+        CD_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, pool, s));
+        return PSB_OK;
     }
-
+    void release(cudaStream_t s) {
+        if (fixed) cudaFreeAsync(fixed, s);
+        if (lists) cudaFreeAsync(lists, s);
+        if (totals) cudaFreeAsync(totals, s);
+        fixed = lists = nullptr;
+        totals = nullptr;
+    }
     ~SegmentEncoder() {
-        cudaFree(x.bsum); cudaFree(x.tot); cudaFree(x.tlen); cudaFree(x.gsum);
-        cudaFree(x.idx); cudaFree(x.blocks); cudaFree(x.refs);
+        if (fixed) cudaFree(fixed);
+        if (lists) cudaFree(lists);
+        if (totals) cudaFree(totals);
     }
 
-    // First half: counts the set bits (chunk prefix sums), cuts them into
-    // blocks of kBlock offsets, finds each block's first and last offset by
-    // select and picks its coding; only StreamVInt blocks get an offset list
-    // and tuple lengths.  Afterwards `count` = offsets, `nb` = blocks,
-    // `bytes` = stream size and hb[b].out_off = block b's offset.
-    // Device buffer for the chunk sums of an n-bit segment (one per kT * 16
-    // words), for a producer that computes them itself (plan(.., true)).
-    int chunk_sums(uint64_t n, unsigned long long** out) {
-        const uint64_t nbs = ((n + 63) / 64 + kT * 16 - 1) / (kT * 16);
-        if (int rc = grow(&x.bsum, &x.cap_bsum, (nbs + 1) * 8)) return rc;
-        *out = x.bsum;
+    static uint64_t chunks(uint64_t n) { return ((n + 63) / 64 + kT * 16 - 1) / (kT * 16); }
+    static uint32_t max_blocks(uint64_t n) { return uint32_t((n + kBlock - 1) / kBlock); }
+
+    int reserve_totals(uint32_t slots, cudaStream_t s) {
+        if (slots <= cap_totals) return PSB_OK;
+        cap_totals = 0;
+        if (int rc = replace(&totals, slots * sizeof(EncTotals), s)) return rc;
+        cap_totals = slots;
+        return PSB_OK;
+    }
+    // Room for segments of n bits.
+    int reserve(uint64_t n, cudaStream_t s) {
+        const size_t at_blocks = ((chunks(n) + 1) * 8 + 255) / 256 * 256;
+        const size_t at_refs = at_blocks + (max_blocks(n) * sizeof(BlockInfo) + 255) / 256 * 256;
+        const size_t need = at_refs + size_t(max_blocks(n)) * 4;
+        if (need > cap_fixed) {
+            cap_fixed = 0;
+            if (int rc = replace(&fixed, need, s)) return rc;
+            cap_fixed = need;
+        }
+        bsum = reinterpret_cast<unsigned long long*>(fixed);
+        blocks = reinterpret_cast<BlockInfo*>(fixed + at_blocks);
+        refs = reinterpret_cast<uint32_t*>(fixed + at_refs);
+        return PSB_OK;
+    }
+    // Room for the offsets of n_refs StreamVInt blocks.
+    int reserve_lists(uint32_t n_refs, cudaStream_t s) {
+        if (n_refs <= cap_refs) return PSB_OK;
+        cap_refs = 0;
+        const size_t at_psum = size_t(n_refs) * kBlock * 4;
+        if (int rc = replace(&lists, at_psum + size_t(n_refs) * kParts * 8, s)) return rc;
+        idx = reinterpret_cast<uint32_t*>(lists);
+        psum = reinterpret_cast<unsigned long long*>(lists + at_psum);
+        cap_refs = n_refs;
         return PSB_OK;
     }
 
-    int plan(const uint64_t* b, uint64_t n, cudaStream_t s, bool sums_ready) {
-        bits = b;
-        n_bits = n;
-        count = tuples = bytes = 0;
-        nb = n_refs = 0;
-        any_bitmap = false;
-        max_words = 1;
-        n_words = (n + 63) / 64;
-        if (n == 0) return PSB_OK;
-        const uint64_t nbs = (n_words + kT * 16 - 1) / (kT * 16);
-        if (int rc = grow(&x.bsum, &x.cap_bsum, (nbs + 1) * 8)) return rc;
-        if (int rc = grow(&x.tot, &x.cap_tot, 8)) return rc;
+    // Counts, cuts and decides the blocks of an n-bit segment (totals[slot]:
+    // count, nb, n_refs).  sums_ready: the chunk popcounts are in bsum.
+    int plan(const uint64_t* bits, uint64_t n, bool sums_ready, uint32_t slot, cudaStream_t s) {
+        const uint64_t n_words = (n + 63) / 64, nbs = chunks(n);
+        EncTotals* t = totals + slot;
         if (!sums_ready) {
-            k_block_sums<<<unsigned(nbs), kT, 0, s>>>(bits, n_words, n_bits, x.bsum);
+            k_block_sums<<<unsigned(nbs), kT, 0, s>>>(bits, n_words, n, bsum);
             launches++;
         }
-        k_scan_small<<<1, kScanT, 0, s>>>(x.bsum, nbs, x.tot);
+        k_scan_small<<<1, kScanT, 0, s>>>(bsum, nbs, &t->count);
+        k_select_blocks<<<std::min(2 * max_blocks(n), kGrid), kT, 0, s>>>(bits, n_words, n, bsum, nbs, t, blocks);
+        k_decide<<<1, kScanT, 0, s>>>(t, blocks, refs, with_ops ? 1 : 0);
+        launches += 3;
+        CD_CUDA(cudaGetLastError());
+        return PSB_OK;
+    }
+    // Lists the StreamVInt blocks' offsets and places the blocks (totals:
+    // bytes, off); `first`: the stream starts at first_off, else after slot - 1's.
+    int layout(const uint64_t* bits, uint64_t n, uint32_t slot, bool first, uint64_t first_off, cudaStream_t s) {
+        EncTotals* t = totals + slot;
+        if (cap_refs) {
+            k_compact<<<unsigned(chunks(n)), kT, 0, s>>>(bits, (n + 63) / 64, n, bsum, chunks(n), t, blocks, cap_refs,
+                                                         idx);
+            k_part_bytes<<<part_grid(n), kT, 0, s>>>(idx, t, blocks, refs, cap_refs, psum);
+            launches += 2;
+        }
+        k_layout<<<1, kScanT, 0, s>>>(t, blocks, psum, cap_refs, with_ops ? 1 : 0, first ? 1 : 0, first_off);
         launches++;
         CD_CUDA(cudaGetLastError());
-        unsigned long long c = 0;
-        CD_CUDA(cudaMemcpyAsync(&c, x.tot, 8, cudaMemcpyDeviceToHost, s));
-        CD_CUDA(cudaStreamSynchronize(s));
-        count = c;
-        if (count == 0) return PSB_OK;  // an empty segment writes nothing (CompressedSegmentWriter)
-        nb = uint32_t((count + kBlock - 1) / kBlock);
-        if (int rc = grow(&x.blocks, &x.cap_blocks, size_t(nb) * sizeof(BlockInfo))) return rc;
-        k_select_blocks<<<2 * nb, kT, 0, s>>>(bits, n_words, n_bits, x.bsum, nbs, count, x.blocks, nb);
-        k_block_decide<<<(nb + kT - 1) / kT, kT, 0, s>>>(count, x.blocks, nb, with_ops ? 1 : 0);
-        launches += 2;
-        CD_CUDA(cudaGetLastError());
-        hb.resize(nb);
-        CD_CUDA(cudaMemcpyAsync(hb.data(), x.blocks, size_t(nb) * sizeof(BlockInfo), cudaMemcpyDeviceToHost, s));
-        CD_CUDA(cudaStreamSynchronize(s));
-        // StreamVInt blocks in order: 2 tuples per 8 values (count padded to a multiple of 8).
-        hrefs.clear();
-        for (uint32_t k = 0; k < nb; k++) {
-            if (hb[k].is_bitmap) {
-                any_bitmap = true;
-                max_words = std::max<uint64_t>(max_words, (uint64_t(hb[k].last) - hb[k].first + 63) / 64);
-                continue;
-            }
-            hrefs.push_back(SviRef{tuples, k, 0});
-            tuples += (uint64_t(hb[k].count) + 7) / 8 * 2;
-        }
-        n_refs = uint32_t(hrefs.size());
-        if (tuples) {
-            if (int rc = grow(&x.refs, &x.cap_refs, size_t(n_refs) * sizeof(SviRef))) return rc;
-            CD_CUDA(cudaMemcpyAsync(x.refs, hrefs.data(), size_t(n_refs) * sizeof(SviRef), cudaMemcpyHostToDevice, s));
-            if (int rc = grow(&x.idx, &x.cap_idx, count * 4)) return rc;
-            k_compact<<<unsigned(nbs), kT, 0, s>>>(bits, n_words, n_bits, x.bsum, nbs, count, x.blocks, x.idx);
-            if (int rc = grow(&x.tlen, &x.cap_tlen, (tuples + 1) * 8)) return rc;
-            k_tuple_len<<<unsigned((tuples + kT - 1) / kT), kT, 0, s>>>(x.idx, x.blocks, x.refs, n_refs, tuples,
-                                                                       x.tlen);
-            CD_CUDA(cudaGetLastError());
-            // Tuple offsets: exclusive scan of the tuple lengths (two levels: groups of 4096).
-            const uint64_t groups = (tuples + kT * 16 - 1) / (kT * 16);
-            if (int rc = grow(&x.gsum, &x.cap_gsum, (groups + 1) * 8)) return rc;
-            k_group_sums<<<unsigned(groups), kT, 0, s>>>(x.tlen, tuples, x.gsum);
-            k_scan_small<<<1, kScanT, 0, s>>>(x.gsum, groups, x.tot);
-            k_group_scan<<<unsigned(groups), kT, 0, s>>>(x.tlen, tuples, x.gsum);
-            unsigned long long svi_total = 0;
-            CD_CUDA(cudaMemcpyAsync(&svi_total, x.tot, 8, cudaMemcpyDeviceToHost, s));
-            CD_CUDA(cudaStreamSynchronize(s));
-            k_block_bytes<<<(n_refs + kT - 1) / kT, kT, 0, s>>>(x.blocks, x.refs, n_refs, x.tlen, tuples, svi_total,
-                                                              with_ops ? 1 : 0);
-            launches += 6;
-            CD_CUDA(cudaGetLastError());
-            CD_CUDA(cudaMemcpyAsync(hb.data(), x.blocks, size_t(nb) * sizeof(BlockInfo), cudaMemcpyDeviceToHost, s));
-            CD_CUDA(cudaStreamSynchronize(s));
-        }
-        unsigned long long off = 0;
-        for (uint32_t k = 0; k < nb; k++) {
-            hb[k].out_off = off;
-            off += hb[k].bytes;
-        }
-        bytes = off;
         return PSB_OK;
     }
-
-    // Second half: writes the planned stream (`bytes` bytes) to d_out.
-    int write(uint8_t* d_out, cudaStream_t s) {
-        if (count == 0) return PSB_OK;
-        CD_CUDA(cudaMemcpyAsync(x.blocks, hb.data(), size_t(nb) * sizeof(BlockInfo), cudaMemcpyHostToDevice, s));
-        if (tuples) {
-            k_write_svi<<<unsigned((tuples + kT - 1) / kT), kT, 0, s>>>(x.idx, x.blocks, x.refs, n_refs, tuples, x.tlen,
-                                                                       d_out);
+    // Writes the stream at out + off if it ends within out_cap bytes of out.
+    int write(const uint64_t* bits, uint64_t n, uint32_t slot, uint8_t* out, uint64_t out_cap, cudaStream_t s) {
+        const EncTotals* t = totals + slot;
+        if (cap_refs) {
+            k_write_svi<<<part_grid(n), kT, 0, s>>>(idx, t, blocks, refs, cap_refs, psum, out, out_cap);
             launches++;
             if (with_ops) {
-                const uint64_t groups = tuples / 2;
-                k_write_bounds<<<unsigned((groups + kT - 1) / kT), kT, 0, s>>>(x.idx, x.blocks, x.refs, n_refs, groups,
-                                                                              ops_nib, ops_first, d_out);
+                k_write_bounds<<<part_grid(n), kT, 0, s>>>(idx, t, blocks, refs, cap_refs, ops_nib, ops_first, out,
+                                                           out_cap);
                 launches++;
             }
         }
-        if (any_bitmap) {
-            k_write_bitmap<<<dim3(unsigned((max_words + kT - 1) / kT), nb), kT, 0, s>>>(
-                bits, n_words, n_bits, x.blocks, x.bsum, (n_words + kT * 16 - 1) / (kT * 16), count, d_out);
+        if (!with_ops) {
+            const unsigned grid = unsigned(std::min<uint64_t>(uint64_t(max_blocks(n)) * kBitmapParts, kGrid));
+            k_write_bitmap<<<grid, kT, 0, s>>>(bits, (n + 63) / 64, n, t, blocks, bsum, chunks(n), cap_refs, out,
+                                               out_cap);
             launches++;
         }
         CD_CUDA(cudaGetLastError());
         return PSB_OK;
+    }
+
+private:
+    static constexpr unsigned kGrid = 148 * 8;  // grids of kernels that loop over items
+    unsigned part_grid(uint64_t n) const {
+        return unsigned(std::min<uint64_t>(uint64_t(std::min(cap_refs, max_blocks(n))) * kParts, kGrid));
     }
 };
 
@@ -783,22 +871,33 @@ __global__ void k_opbits_decode(const uint8_t* __restrict__ in, uint64_t groups,
 SegmentEncoder* encoder_create() { return new (std::nothrow) SegmentEncoder(); }
 void encoder_destroy(SegmentEncoder* e) { delete e; }
 
-int encoder_chunk_sums(SegmentEncoder* e, uint64_t n_bits, unsigned long long** sums) {
-    return e->chunk_sums(n_bits, sums);
-}
-
-int encoder_plan(SegmentEncoder* e, const uint64_t* d_bits, uint64_t n_bits, cudaStream_t s, bool sums_ready,
-                 uint64_t* bytes, uint64_t* count) {
-    if (int rc = e->plan(d_bits, n_bits, s, sums_ready)) return rc;
-    *bytes = e->bytes;
-    *count = e->count;
+int encoder_begin(SegmentEncoder* e, uint64_t n_bits, uint32_t slots, cudaStream_t s, unsigned long long** sums) {
+    if (int rc = e->reserve(n_bits, s)) return rc;
+    if (int rc = e->reserve_totals(slots, s)) return rc;
+    *sums = e->bsum;
     return PSB_OK;
 }
 
-int encoder_write(SegmentEncoder* e, uint8_t* d_out, cudaStream_t s) { return e->write(d_out, s); }
+int encoder_segment(SegmentEncoder* e, const uint64_t* d_bits, uint64_t n_bits, bool sums_ready, uint32_t slot,
+                    uint64_t first_off, uint8_t* out, uint64_t out_cap, cudaStream_t s) {
+    if (int rc = e->plan(d_bits, n_bits, sums_ready, slot, s)) return rc;
+    if (int rc = e->layout(d_bits, n_bits, slot, slot == 0, first_off, s)) return rc;
+    return e->write(d_bits, n_bits, slot, out, out_cap, s);
+}
+
+int encoder_totals(SegmentEncoder* e, uint32_t slots, EncTotals* host, bool* complete, cudaStream_t s) {
+    CD_CUDA(cudaMemcpyAsync(host, e->totals, slots * sizeof(EncTotals), cudaMemcpyDeviceToHost, s));
+    CD_CUDA(cudaStreamSynchronize(s));
+    uint32_t most = 0;
+    for (uint32_t i = 0; i < slots; ++i) most = std::max(most, host[i].n_refs);
+    *complete = most <= e->cap_refs;
+    return *complete ? PSB_OK : e->reserve_lists(most + most / 4, s);
+}
 
 void encoder_set_ops(SegmentEncoder* e, bool on, const uint64_t* nibbles, uint64_t first_state) {
-    e->set_ops(on, nibbles, first_state);
+    e->with_ops = on;
+    e->ops_nib = nibbles;
+    e->ops_first = first_state;
 }
 
 uint64_t encoder_take_launches(SegmentEncoder* e) {
@@ -818,20 +917,35 @@ extern "C" int psb_frontier_encode(const uint64_t* d_bits, uint64_t first_bit, u
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     *out_bytes = 0;
     *n_blocks = 0;
+    if (n_bits == 0) return PSB_OK;
+    const uint64_t* bits = d_bits + first_bit / 64;
     psb::SegmentEncoder E;
-    if (int rc = E.plan(d_bits + first_bit / 64, n_bits, s, false)) return rc;
-    *out_bytes = E.bytes;
-    *n_blocks = E.nb;
-    if (E.count == 0) return PSB_OK;
-    if (blocks) {
-        if (blocks_cap < E.nb) return psb_set_error(PSB_ERR_CAPACITY, "blocks table too small");
-        for (uint32_t b = 0; b < E.nb; b++)
-            blocks[b] = psb_codec_block{E.hb[b].out_off, E.hb[b].count, uint32_t(E.hb[b].bytes), E.hb[b].first,
-                                        E.hb[b].is_bitmap};
-    }
-    if (!d_out || out_cap < E.bytes) return psb_set_error(PSB_ERR_CAPACITY, "output needs more bytes (see *out_bytes)");
-    if (int rc = E.write(d_out, s)) return rc;
+    // Scratch goes back to the pool in stream order, whatever the outcome.
+    struct Release { psb::SegmentEncoder& e; cudaStream_t s; ~Release() { e.release(s); } } release{E, s};
+    if (int rc = E.reserve(n_bits, s)) return rc;
+    if (int rc = E.reserve_totals(1, s)) return rc;
+    if (int rc = E.plan(bits, n_bits, false, 0, s)) return rc;
+    EncTotals t{};
+    CD_CUDA(cudaMemcpyAsync(&t, E.totals, sizeof t, cudaMemcpyDeviceToHost, s));
     CD_CUDA(cudaStreamSynchronize(s));
+    if (t.count == 0) return PSB_OK;  // an empty segment writes nothing (CompressedSegmentWriter)
+    // The offset list has its exact size now.
+    if (int rc = E.reserve_lists(t.n_refs, s)) return rc;
+    if (int rc = E.layout(bits, n_bits, 0, true, 0, s)) return rc;
+    const bool table = blocks && blocks_cap >= t.nb;
+    if (d_out && (!blocks || table))  // written only if it fits
+        if (int rc = E.write(bits, n_bits, 0, d_out, out_cap, s)) return rc;
+    std::vector<BlockInfo> hb(table ? t.nb : 0);
+    if (table)
+        CD_CUDA(cudaMemcpyAsync(hb.data(), E.blocks, hb.size() * sizeof(BlockInfo), cudaMemcpyDeviceToHost, s));
+    CD_CUDA(cudaMemcpyAsync(&t, E.totals, sizeof t, cudaMemcpyDeviceToHost, s));
+    CD_CUDA(cudaStreamSynchronize(s));
+    *out_bytes = t.bytes;
+    *n_blocks = t.nb;
+    if (blocks && !table) return psb_set_error(PSB_ERR_CAPACITY, "blocks table too small");
+    for (size_t b = 0; b < hb.size(); b++)
+        blocks[b] = psb_codec_block{hb[b].out_off, hb[b].count, uint32_t(hb[b].bytes), hb[b].first, hb[b].is_bitmap};
+    if (!d_out || out_cap < t.bytes) return psb_set_error(PSB_ERR_CAPACITY, "output needs more bytes (see *out_bytes)");
     return PSB_OK;
 }
 

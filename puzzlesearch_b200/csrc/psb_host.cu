@@ -803,6 +803,8 @@ struct SpillSeg {
     uint64_t off, bytes, states;
 };
 
+constexpr uint32_t kSpillBatch = 256;  // segments encoded between two waits
+
 struct SpillSlot {
     uint8_t* host = nullptr;
     uint64_t host_cap = 0;
@@ -818,6 +820,7 @@ struct SpillRes {
     uint64_t arena_cap = 0;  // bytes
     std::vector<SpillSeg> segs;  // the depth in the arena
     std::vector<uint8_t> flags;  // host copy of the depth's active-window flags
+    psb::EncTotals* totals = nullptr;  // a batch of segments' sizes (pinned)
     size_t issued = 0, delivered = 0;
     SpillSlot slot[2];  // segment i goes through slot i % 2
     cudaStream_t copy = nullptr;
@@ -832,6 +835,7 @@ struct SpillRes {
         }
         cudaFree(bits);
         cudaFree(arena);
+        if (totals) cudaFreeHost(totals);
         if (enc) psb::encoder_destroy(enc);
         if (encoded) cudaEventDestroy(encoded);
         if (copy) cudaStreamDestroy(copy);
@@ -861,6 +865,7 @@ int spill_acquire(int device, SpillRes** out) {
     std::unique_ptr<SpillRes> R(new (std::nothrow) SpillRes());
     if (!R || !(R->enc = psb::encoder_create())) return fail(PSB_ERR_NOMEM, "spill resources");
     R->device = device;
+    PSB_CUDA(cudaMallocHost(&R->totals, kSpillBatch * sizeof(psb::EncTotals)));
     PSB_CUDA(cudaStreamCreateWithFlags(&R->copy, cudaStreamNonBlocking));
     PSB_CUDA(cudaEventCreateWithFlags(&R->encoded, cudaEventDisableTiming));
     for (auto& sl : R->slot) {
@@ -1114,64 +1119,76 @@ int spill_depth(psb_bfs_session* S, const psb_bfs_opts* o, uint32_t depth, const
     SpillRes* R = S->spill;
     R->segs.clear();
     R->issued = R->delivered = 0;
-    if (src.flags) {
+    if (src.flags && N > seg) {  // which segments can hold states
         R->flags.resize(src.n_windows);
         PSB_CUDA(cudaMemcpyAsync(R->flags.data(), src.flags, src.n_windows, cudaMemcpyDeviceToHost, s));
         PSB_CUDA(cudaStreamSynchronize(s));
     }
+    // The segments are enqueued back to back, up to kSpillBatch of them, and
+    // waited for once; a batch whose streams or offset lists outgrow their
+    // buffers is encoded again in larger ones (its arrays have not changed).
+    struct OpsOff { psb::SegmentEncoder* e; ~OpsOff() { psb::encoder_set_ops(e, false, nullptr, 0); } } ops_off{R->enc};
     uint64_t off = 0;
-    for (uint64_t g = 0; g * seg < N; g++) {
-        const uint64_t first = g * seg, n = std::min(seg, N - first);
-        if (src.flags) {
-            const uint64_t w0 = first >> src.window_bits, w1 = std::min(src.n_windows, ((first + n - 1) >> src.window_bits) + 1);
-            if (std::find_if(R->flags.begin() + w0, R->flags.begin() + w1, [](uint8_t f) { return f != 0; }) ==
-                R->flags.begin() + w1)
-                continue;
-        }
-        bool sums_ready = false;  // the extraction kernels also count
-        if (!src.bitmap) {
-            if (src.single != PSB_INVALID_INDEX && (src.single < first || src.single - first >= n)) continue;
-            const uint64_t words = (n + 63) / 64;
-            if (int rc = grow_device(&R->bits, &R->bits_cap, words * 8)) return rc;
-            if (src.single != PSB_INVALID_INDEX) {
-                PSB_CUDA(cudaMemsetAsync(R->bits, 0, words * 8, s));
-                if (int rc = set_bit(R->bits, src.single - first, s)) return rc;
-            } else {
-                unsigned long long* sums = nullptr;
-                if (int rc = psb::encoder_chunk_sums(R->enc, n, &sums)) return rc;
-                t->launches++;
-                const int rc =
-                    src.codes ? psb::frontier_bits_two_bit(src.codes, first, n, src.code, R->bits, sums, src.flags,
-                                                           src.window_bits, src.n_windows, s)
-                              : psb::frontier_bits_nibbles(src.nibbles, src.excl, first, n, R->bits, sums, s);
-                if (rc) return rc;
-                sums_ready = true;
+    for (uint64_t g = 0; g * seg < N;) {
+        unsigned long long* sums = nullptr;
+        const uint64_t g0 = g, off0 = off;
+        uint32_t batch[kSpillBatch], slots = 0;
+        if (int rc = psb::encoder_begin(R->enc, std::min(seg, N), kSpillBatch, s, &sums)) return rc;
+        for (; g * seg < N && slots < kSpillBatch; g++) {
+            const uint64_t first = g * seg, n = std::min(seg, N - first);
+            if (src.flags && N > seg) {
+                const uint64_t w0 = first >> src.window_bits, w1 = std::min(src.n_windows, ((first + n - 1) >> src.window_bits) + 1);
+                if (std::find_if(R->flags.begin() + w0, R->flags.begin() + w1, [](uint8_t f) { return f != 0; }) ==
+                    R->flags.begin() + w1)
+                    continue;
             }
+            bool sums_ready = false;  // the extraction kernels also count
+            if (!src.bitmap) {
+                if (src.single != PSB_INVALID_INDEX && (src.single < first || src.single - first >= n)) continue;
+                const uint64_t words = (n + 63) / 64;
+                if (int rc = grow_device(&R->bits, &R->bits_cap, words * 8)) return rc;
+                if (src.single != PSB_INVALID_INDEX) {
+                    PSB_CUDA(cudaMemsetAsync(R->bits, 0, words * 8, s));
+                    if (int rc = set_bit(R->bits, src.single - first, s)) return rc;
+                } else {
+                    t->launches++;
+                    const int rc =
+                        src.codes ? psb::frontier_bits_two_bit(src.codes, first, n, src.code, R->bits, sums, src.flags,
+                                                               src.window_bits, src.n_windows, s)
+                                  : psb::frontier_bits_nibbles(src.nibbles, src.excl, first, n, R->bits, sums, s);
+                    if (rc) return rc;
+                    sums_ready = true;
+                }
+            }
+            const uint64_t* bits = src.bitmap ? src.bitmap + first / 64 : R->bits;  // after the scratch exists
+            psb::encoder_set_ops(R->enc, src.ops, src.nibbles, first);  // the initial state's nibble is 0
+            if (int rc = psb::encoder_segment(R->enc, bits, n, sums_ready, slots, off, R->arena, R->arena_cap, s)) return rc;
+            batch[slots++] = uint32_t(g);
         }
-        const uint64_t* bits = src.bitmap ? src.bitmap + first / 64 : R->bits;  // after the scratch exists
-        uint64_t bytes = 0, count = 0;
-        psb::encoder_set_ops(R->enc, src.ops, src.nibbles, first);  // the initial state's nibble is 0
-        const int prc = psb::encoder_plan(R->enc, bits, n, s, sums_ready, &bytes, &count);
-        if (prc) {
-            psb::encoder_set_ops(R->enc, false, nullptr, 0);
-            return prc;
+        if (slots == 0) continue;
+        bool complete = false;
+        if (int rc = psb::encoder_totals(R->enc, slots, R->totals, &complete, s)) return rc;
+        const uint64_t end = R->totals[slots - 1].off + R->totals[slots - 1].bytes;
+        if (!complete || end > R->arena_cap) {
+            if (complete) {  // grow, keeping this depth's segments written so far
+                const uint64_t want = end + end / 4;
+                uint8_t* bigger = nullptr;
+                PSB_CUDA(cudaMalloc(reinterpret_cast<void**>(&bigger), want));
+                if (off0) PSB_CUDA(cudaMemcpyAsync(bigger, R->arena, off0, cudaMemcpyDeviceToDevice, s));
+                PSB_CUDA(cudaStreamSynchronize(s));
+                PSB_CUDA(cudaFree(R->arena));
+                R->arena = bigger;
+                R->arena_cap = want;
+            }
+            g = g0;  // the batch again
+            off = off0;
+            continue;
         }
-        if (count == 0) continue;
-        if (R->arena_cap < off + bytes) {  // grow, keeping this depth's segments written so far
-            const uint64_t want = (off + bytes) + (off + bytes) / 4;
-            uint8_t* bigger = nullptr;
-            PSB_CUDA(cudaMalloc(reinterpret_cast<void**>(&bigger), want));
-            if (off) PSB_CUDA(cudaMemcpyAsync(bigger, R->arena, off, cudaMemcpyDeviceToDevice, s));
-            PSB_CUDA(cudaStreamSynchronize(s));
-            PSB_CUDA(cudaFree(R->arena));
-            R->arena = bigger;
-            R->arena_cap = want;
+        for (uint32_t i = 0; i < slots; i++) {
+            const psb::EncTotals& e = R->totals[i];
+            if (e.count) R->segs.push_back(SpillSeg{depth, batch[i], e.off, e.bytes, e.count});
         }
-        const int wrc = psb::encoder_write(R->enc, R->arena + off, s);
-        psb::encoder_set_ops(R->enc, false, nullptr, 0);
-        if (wrc) return wrc;
-        R->segs.push_back(SpillSeg{depth, uint32_t(g), off, bytes, count});
-        off += bytes;
+        off = end;
     }
     t->launches += psb::encoder_take_launches(R->enc);
     PSB_CUDA(cudaEventRecord(R->encoded, s));

@@ -45,24 +45,35 @@ __global__ void retire_two_bit(ulonglong2* __restrict__ codes, uint64_t n2, uint
                                unsigned long long* count);
 
 // Frontier encoder with device scratch kept between segments (psb_codec.cu).
+// Segments are encoded in stream order without waiting for the device: each
+// leaves its sizes in a totals slot, read back for all of them at once.
+struct EncTotals {
+    unsigned long long count;  // offsets
+    unsigned long long bytes;  // of the stream
+    unsigned long long off;    // its place in the output
+    uint32_t nb, n_refs;       // blocks, StreamVInt blocks among them
+};
 struct SegmentEncoder;
 SegmentEncoder* encoder_create();
 void encoder_destroy(SegmentEncoder* e);
-// Plans the reference's segment stream of the set bits of d_bits[0, n_bits)
-// (n_bits <= 2^32): *count offsets in *bytes bytes; encoder_write then
-// writes it to d_out (device, >= *bytes).  d_bits must stay unchanged
-// until the write has run (both are ordered on stream s).  sums_ready: the
-// chunk popcounts are already in encoder_chunk_sums' buffer.
-int encoder_plan(SegmentEncoder* e, const uint64_t* d_bits, uint64_t n_bits, cudaStream_t s, bool sums_ready,
-                 uint64_t* bytes, uint64_t* count);
-int encoder_write(SegmentEncoder* e, uint8_t* d_out, cudaStream_t s);
+// Scratch for segments of up to n_bits bits (<= 2^32) and `slots` totals;
+// *sums is the chunk-popcount buffer a producer of bitmaps may fill.
+int encoder_begin(SegmentEncoder* e, uint64_t n_bits, uint32_t slots, cudaStream_t s, unsigned long long** sums);
+// Enqueues one segment: the reference's segment stream of the set bits of
+// d_bits[0, n_bits), at out + first_off (slot 0) or after slot - 1's stream,
+// if it ends within out_cap.  d_bits must stay unchanged until the write has
+// run.  sums_ready: the chunk popcounts are already in encoder_begin's buffer.
+int encoder_segment(SegmentEncoder* e, const uint64_t* d_bits, uint64_t n_bits, bool sums_ready, uint32_t slot,
+                    uint64_t first_off, uint8_t* out, uint64_t out_cap, cudaStream_t s);
+// Waits for the segments and reads their totals.  *complete false: some
+// segment needed a longer offset list, which is there now; all have to be
+// enqueued again.  A segment whose off + bytes exceed out_cap was not written.
+int encoder_totals(SegmentEncoder* e, uint32_t slots, EncTotals* host, bool* complete, cudaStream_t s);
 // Frontier-search segments carry each state's operator bits: with `on`, the
-// following plans write CompressedFrontierWriter's stream (StreamVInt blocks
+// following segments are CompressedFrontierWriter's streams (StreamVInt blocks
 // with bounds, Common/CompressedFrontier.cpp:63-70) whose nibble for offset v
 // is state first_state + v of `nibbles` (a 4-bit array; NULL = all zero).
 void encoder_set_ops(SegmentEncoder* e, bool on, const uint64_t* nibbles, uint64_t first_state);
-// The encoder's chunk-sum buffer sized for an n_bits segment.
-int encoder_chunk_sums(SegmentEncoder* e, uint64_t n_bits, unsigned long long** sums);
 // Kernels the encoder launched since the last call.
 uint64_t encoder_take_launches(SegmentEncoder* e);
 // Segment store (psb_store.cu): the reference's Store over files in some
@@ -95,7 +106,7 @@ int frontier_decode_async(const uint8_t* d_in, const psb_codec_block* h_blocks, 
 // One-bit frontier bitmaps (ceil(n_states/64) words at out; first_state a
 // multiple of 64) of a two-bit array (states with code `code`) and of a
 // frontier-search array (states with an operator bit set, less `excl`),
-// with their chunk popcounts in `sums` (from encoder_chunk_sums).  Two-bit
+// with their chunk popcounts in `sums` (from encoder_begin).  Two-bit
 // extraction may be given the depth's active-window flags (NULL = none):
 // chunks of unflagged windows count 0 and are not written.
 int frontier_bits_two_bit(const uint64_t* codes, uint64_t first_state, uint64_t n_states, uint32_t code,

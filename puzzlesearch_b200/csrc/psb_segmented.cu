@@ -173,11 +173,21 @@ struct Run {
     // Encodes a segment bitmap holding `count` states as segment g's layer in `store`.
     int encode(const uint64_t* bits, uint64_t g, uint64_t count, psb::StoreImpl& store) {
         if (count == 0) return PSB_OK;
-        uint64_t bytes = 0, n = 0;
-        if (int rc = psb::encoder_plan(enc, bits, states_in(g), s, false, &bytes, &n)) return rc;
-        if (n != count) return psb_set_error(PSB_ERR_DEVICE, "segmented search: layer count mismatch");
-        if (int rc = stream_buf[0].grow(bytes)) return rc;
-        if (int rc = psb::encoder_write(enc, stream_buf[0].p, s)) return rc;
+        unsigned long long* sums = nullptr;
+        if (int rc = psb::encoder_begin(enc, std::min(seg_states, P->n_states), 1, s, &sums)) return rc;
+        psb::EncTotals t{};
+        for (;;) {  // again with longer buffers if the segment outgrows them
+            if (int rc = psb::encoder_segment(enc, bits, states_in(g), false, 0, 0, stream_buf[0].p,
+                                              stream_buf[0].cap, s))
+                return rc;
+            bool complete = false;
+            if (int rc = psb::encoder_totals(enc, 1, &t, &complete, s)) return rc;
+            if (complete && t.bytes <= stream_buf[0].cap) break;
+            if (complete)
+                if (int rc = stream_buf[0].grow(t.bytes)) return rc;
+        }
+        const uint64_t bytes = t.bytes;
+        if (t.count != count) return psb_set_error(PSB_ERR_DEVICE, "segmented search: layer count mismatch");
         if (host_stream.size() < bytes) host_stream.resize(bytes);
         SG_CUDA(cudaMemcpyAsync(host_stream.data(), stream_buf[0].p, bytes, cudaMemcpyDeviceToHost, s));
         SG_CUDA(cudaStreamSynchronize(s));
