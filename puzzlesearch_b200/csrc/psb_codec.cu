@@ -33,6 +33,8 @@ namespace {
 constexpr uint32_t kBlock = 256 * 1024;  // StreamVInt::MAX_INDEXES_COUNT (Common/StreamVInt.h:9)
 constexpr uint32_t kMap = 0x80000000u;   // CODEC_MAP (Common/FrontierCompression.cpp:6)
 constexpr int kT = 256;
+constexpr int kCW = 4;                      // words per thread of a chunk
+constexpr uint32_t kChunkWords = kT * kCW;  // bitmap words whose popcounts are summed together
 
 #define CD_CUDA(call)                                                                           \
     do {                                                                                        \
@@ -48,11 +50,12 @@ __device__ __forceinline__ uint64_t masked_word(const uint64_t* bits, uint64_t w
     return v;
 }
 
-// Per-block sums of word popcounts (kT threads x 16 words per block).
+// Popcount of each chunk of kChunkWords words.
 __global__ void k_block_sums(const uint64_t* bits, uint64_t n_words, uint64_t n_bits, unsigned long long* bsum) {
-    const uint64_t base = uint64_t(blockIdx.x) * kT * 16;
+    const uint64_t base = uint64_t(blockIdx.x) * kChunkWords;
     uint32_t c = 0;
-    for (int k = 0; k < 16; ++k) {
+#pragma unroll
+    for (int k = 0; k < kCW; ++k) {
         const uint64_t w = base + uint64_t(k) * kT + threadIdx.x;
         if (w < n_words) c += __popcll(masked_word(bits, w, n_words, n_bits));
     }
@@ -157,7 +160,7 @@ struct BlockInfo {
 using psb::EncTotals;
 
 // StreamVInt blocks are worked on in parts of kPartTuples tuples.
-constexpr uint32_t kPartTuples = 4096, kParts = kBlock / 4 / kPartTuples;
+constexpr uint32_t kPartTuples = 1024, kParts = kBlock / 4 / kPartTuples;
 // Bitmap blocks in parts of kPartWords words: a bitmap block's bitmap is
 // smaller than 10 bits per offset, so 40 parts hold any.
 constexpr uint32_t kPartWords = 1024, kBitmapParts = 40;
@@ -165,82 +168,91 @@ static_assert(uint64_t(kBitmapParts) * kPartWords * 64 >= uint64_t(kBlock) * 10,
 
 // Writes the ascending offsets of the set bits that fall in StreamVInt
 // blocks into their block's place of the offset list (bitmap blocks need no
-// list: their words are copied from the bitmap).  One CTA per chunk of
-// kT * 16 words; warp w takes the chunk's words 512 w .. 512 w + 511, 32 at a
-// time, lane l word 32 i + l, so every load is coalesced.  A first pass
-// counts each warp's offsets (one CTA scan of the 8 warp totals gives the
-// warps' first ranks); the second pass reloads the words (from L1) and ranks
-// each lane's offsets by a warp scan, so neighbouring lanes store
-// neighbouring ranks.
+// list: their words are copied from the bitmap).  One CTA per chunk; warp w
+// takes words 128 w .. 128 w + 127 of it, lane l words l, 32 + l, .. of those
+// (a dense stretch is spread over the lanes), and two scans of paired counts
+// rank all of the warp's offsets.  The lanes put them into shared memory at
+// their ranks and the warp stores them in order; a warp with more than
+// kStaged offsets stores each where it goes.
+// (A rank-ordered search per 32 words took 52 us where this takes 6: its
+// chain of shuffles, on chunks four times as large.)
+constexpr uint32_t kStaged = 1024;
 __global__ void __launch_bounds__(kT) k_compact(const uint64_t* bits, uint64_t n_words, uint64_t n_bits,
                                                 const unsigned long long* bsum, uint64_t nbs, const EncTotals* totals,
                                                 const BlockInfo* blocks, uint32_t cap_refs, uint32_t* idx) {
     __shared__ uint32_t warp_tot[kT / 32];
+    __shared__ uint16_t staged[kT / 32][kStaged];
     if (totals->n_refs == 0 || totals->n_refs > cap_refs) return;
     // Chunks with no offsets, or whose offsets all fall in bitmap blocks,
-    // have nothing to list (uniform over the CTA: the chunk's rank range).
+    // have nothing to list (uniform over the CTA).  A chunk has at most 65,536
+    // offsets, so they fall in at most two blocks.
     const unsigned long long r_lo = bsum[blockIdx.x];
     const unsigned long long r_hi = blockIdx.x + 1 < nbs ? bsum[blockIdx.x + 1] : totals->count;
     if (r_hi == r_lo) return;
-    bool all_bitmap = true;
-    for (uint64_t b = r_lo / kBlock; b <= (r_hi - 1) / kBlock; ++b) all_bitmap = all_bitmap && blocks[b].is_bitmap;
-    if (all_bitmap) return;
+    const uint64_t b0 = r_lo / kBlock, b1 = (r_hi - 1) / kBlock;
+    const bool list0 = !blocks[b0].is_bitmap, list1 = !blocks[b1].is_bitmap;
+    if (!list0 && !list1) return;
+    uint32_t* const to0 = idx + uint64_t(blocks[b0].svi) * kBlock;
+    uint32_t* const to1 = idx + uint64_t(blocks[b1].svi) * kBlock;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t w0 = uint64_t(blockIdx.x) * kT * 16 + uint64_t(warp) * 512 + lane;
-    uint32_t c = 0;
-#pragma unroll 4
-    for (int i = 0; i < 16; ++i) {
-        const uint64_t w = w0 + 32u * i;
-        if (w < n_words) c += __popcll(masked_word(bits, w, n_words, n_bits));
-    }
-    // The CTA's ranks, warp by warp (warp order is word order).
-    const uint32_t wsum = __reduce_add_sync(0xFFFFFFFFu, c);
-    if (lane == 0) warp_tot[warp] = wsum;
-    __syncthreads();
-    unsigned long long r = r_lo;
-    for (uint32_t k = 0; k < warp; ++k) r += warp_tot[k];
-    if (wsum == 0) return;
-    for (int i = 0; i < 16; ++i) {
-        const uint64_t w = w0 + 32u * i;
-        uint64_t m = w < n_words ? masked_word(bits, w, n_words, n_bits) : 0;
-        const uint32_t cnt = __popcll(m);
-        uint32_t incl = cnt;
+    const uint64_t w0 = uint64_t(blockIdx.x) * kChunkWords + warp * (32 * kCW);  // the warp's first word
+    static_assert(kCW == 4, "two pairs of words per lane");
+    uint64_t v[kCW];
+    uint32_t at[kCW];  // rank of the word's first offset in the warp
+    uint32_t before = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t c = 0;  // counts of words 2h (low half) and 2h + 1; a word row has at most 2048
+#pragma unroll
+        for (int k = 2 * h; k < 2 * h + 2; ++k) {
+            const uint64_t w = w0 + 32 * k + lane;
+            v[k] = w < n_words ? masked_word(bits, w, n_words, n_bits) : 0;
+            c |= uint32_t(__popcll(v[k])) << (16 * (k & 1));
+        }
+        uint32_t incl = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
             if (lane >= uint32_t(o)) incl += y;
         }
-        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        // The 32 words' offsets in rank order, 32 at a time: lane l stores
-        // rank r + k, k = base + l, so a warp's stores are contiguous.
-        for (uint32_t base = 0; base < total; base += 32) {
-            const uint32_t k = base + lane;
-            uint32_t lo = 0, hi = 31;  // source lane: the first whose inclusive count exceeds k
+        const uint32_t rows = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        at[2 * h] = before + (incl & 0xFFFFu) - (c & 0xFFFFu);
+        at[2 * h + 1] = before + (rows & 0xFFFFu) + (incl >> 16) - (c >> 16);
+        before += (rows & 0xFFFFu) + (rows >> 16);
+    }
+    if (lane == 31) warp_tot[warp] = before;
+    __syncthreads();
+    const uint32_t total = warp_tot[warp];
+    unsigned long long r = r_lo;  // rank of the warp's first offset
+    for (uint32_t k = 0; k < warp; ++k) r += warp_tot[k];
+    auto put = [&](uint32_t k, uint32_t offset) {  // the warp's k-th offset
+        const unsigned long long rank = r + k;
+        const bool second = rank / kBlock != b0;
+        if (second ? list1 : list0) (second ? to1 : to0)[rank % kBlock] = offset;
+    };
+    const uint32_t first = uint32_t(w0 * 64);  // offsets fit 32 bits
 #pragma unroll
-            for (int step = 0; step < 5; ++step) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (__shfl_sync(0xFFFFFFFFu, incl, int(mid)) > k) hi = mid;
-                else lo = mid + 1;
-            }
-            const uint32_t before = __shfl_sync(0xFFFFFFFFu, incl - cnt, int(lo));
-            const uint64_t word = __shfl_sync(0xFFFFFFFFu, m, int(lo));
-            if (k < total) {
-                const unsigned long long rank = r + k;
-                const BlockInfo& b = blocks[rank / kBlock];
-                if (!b.is_bitmap)
-                    idx[uint64_t(b.svi) * kBlock + rank % kBlock] =
-                        uint32_t((w0 + 32u * i - lane + lo) * 64 + psb::select_bit(word, k - before));
-            }
+    for (int k = 0; k < kCW; ++k) {
+        uint64_t m = v[k];
+        while (m) {
+            const uint32_t o = (32 * k + lane) * 64 + uint32_t(__ffsll((long long)m) - 1);
+            m &= m - 1;
+            if (total <= kStaged) staged[warp][at[k]] = uint16_t(o);
+            else put(at[k], first + o);
+            ++at[k];
         }
-        r += total;
+    }
+    if (total <= kStaged) {
+        __syncwarp();
+        for (uint32_t k = lane; k < total; k += 32) put(k, first + staged[warp][k]);
     }
 }
 
 // First and last offset of every block (ranks b * kBlock and the block's
 // last rank), by select: the chunk holding the rank from the chunk prefix
-// sums (bsum, chunks of kT * 16 words), then a block scan of that chunk's
-// per-thread counts (thread t: words 16 t .. 16 t + 15).  Items 2b and 2b + 1
-// serve block b.
+// sums (a search with one probe per thread a turn), then a block scan of that
+// chunk's per-thread counts (thread t: words kCW t .. kCW t + kCW - 1).  Items
+// 2b and 2b + 1 serve block b.
 __global__ void __launch_bounds__(kT) k_select_blocks(const uint64_t* bits, uint64_t n_words, uint64_t n_bits,
                                                       const unsigned long long* bsum, uint64_t nbs,
                                                       const EncTotals* totals, BlockInfo* blocks) {
@@ -251,17 +263,19 @@ __global__ void __launch_bounds__(kT) k_select_blocks(const uint64_t* bits, uint
         const bool last = item & 1;
         const uint64_t end = (b + 1) * kBlock < count ? (b + 1) * kBlock : count;
         const uint64_t r = last ? end - 1 : b * kBlock;
-        uint64_t lo = 0, hi = nbs;  // largest chunk lo with bsum[lo] <= r (bsum[0] = 0)
-        while (hi - lo > 1) {
-            const uint64_t mid = (lo + hi) / 2;
-            if (bsum[mid] <= r) lo = mid; else hi = mid;
+        uint64_t lo = 0, n = nbs;  // the largest chunk with bsum <= r is in [lo, lo + n) (bsum[0] = 0)
+        while (n > 1) {
+            const uint64_t step = (n + kT - 1) / kT, at = threadIdx.x * step;
+            const uint32_t k = __syncthreads_count(at < n && bsum[lo + at] <= r);
+            lo += (k - 1) * step;
+            n = n - (k - 1) * step < step ? n - (k - 1) * step : step;
         }
         const uint64_t rem = r - bsum[lo];
-        const uint64_t w0 = lo * kT * 16 + uint64_t(threadIdx.x) * 16;
-        uint64_t v[16];
+        const uint64_t w0 = lo * kChunkWords + uint64_t(threadIdx.x) * kCW;
+        uint64_t v[kCW];
         uint32_t c = 0;
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
+        for (int k = 0; k < kCW; ++k) {
             v[k] = w0 + k < n_words ? masked_word(bits, w0 + k, n_words, n_bits) : 0;
             c += __popcll(v[k]);
         }
@@ -270,7 +284,7 @@ __global__ void __launch_bounds__(kT) k_select_blocks(const uint64_t* bits, uint
         if (rem < exc || rem >= inc) continue;  // exactly one thread holds the rank
         uint32_t left = uint32_t(rem - exc);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
+        for (int k = 0; k < kCW; ++k) {
             const uint32_t ck = __popcll(v[k]);
             if (left < ck) {
                 const uint32_t pos = uint32_t((w0 + k) * 64 + psb::select_bit(v[k], left));
@@ -382,31 +396,35 @@ __global__ void __launch_bounds__(kT) k_part_bytes(const uint32_t* idx, const En
 // parts' first bytes (psum becomes their exclusive prefix), each block's
 // offset in the stream and the segment's place: at `first_off`, or after the
 // segment before it.  One CTA.
-__global__ void __launch_bounds__(kScanT) k_layout(EncTotals* totals, BlockInfo* blocks, unsigned long long* psum,
-                                                   uint32_t cap_refs, int with_ops, int first,
+__global__ void __launch_bounds__(kScanT) k_layout(EncTotals* totals, BlockInfo* blocks, const uint32_t* refs,
+                                                   unsigned long long* psum, uint32_t cap_refs, int with_ops, int first,
                                                    unsigned long long first_off) {
     __shared__ unsigned long long warp_tot[kScanT / 32];
     const uint64_t nb = totals->nb;
-    const bool listed = totals->n_refs <= cap_refs;
+    const uint32_t n_refs = totals->n_refs <= cap_refs ? totals->n_refs : 0;  // the listed ones
+    // A warp per StreamVInt block: its parts' bytes, two per lane.
+    static_assert(kParts == 64, "two parts per lane");
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t ref = threadIdx.x >> 5; ref < n_refs; ref += kScanT / 32) {
+        ulonglong2* parts = reinterpret_cast<ulonglong2*>(psum + uint64_t(ref) * kParts) + lane;
+        const ulonglong2 own = *parts;
+        unsigned long long incl = own.x + own.y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= uint32_t(o)) incl += y;
+        }
+        *parts = make_ulonglong2(incl - own.x - own.y, incl - own.y);
+        if (lane == 31) {
+            BlockInfo& bi = blocks[refs[ref]];
+            bi.bytes = 4 + incl + (with_ops ? (uint64_t(bi.count) + 7) / 8 * 4 : 0);
+        }
+    }
+    __syncthreads();
     unsigned long long off = 0;
     for (uint64_t b0 = 0; b0 < nb; b0 += kScanT) {
         const uint64_t b = b0 + threadIdx.x;
-        unsigned long long bytes = 0;
-        if (b < nb) {
-            BlockInfo& bi = blocks[b];
-            if (!bi.is_bitmap) {
-                unsigned long long t = 0;
-                if (listed) {
-                    for (uint32_t p = 0; p < kParts; ++p) {
-                        const unsigned long long own = psum[uint64_t(bi.svi) * kParts + p];
-                        psum[uint64_t(bi.svi) * kParts + p] = t;
-                        t += own;
-                    }
-                }
-                bi.bytes = 4 + t + (with_ops ? (uint64_t(bi.count) + 7) / 8 * 4 : 0);
-            }
-            bytes = bi.bytes;
-        }
+        const unsigned long long bytes = b < nb ? blocks[b].bytes : 0;
         unsigned long long total;
         const unsigned long long incl = scan_cta(bytes, warp_tot, &total);
         if (b < nb) blocks[b].out_off = off + incl - bytes;
@@ -522,11 +540,11 @@ __global__ void __launch_bounds__(kT) k_write_bounds(const uint32_t* idx, const 
 }
 
 // Bitmap block: bit j of output word i is state first + 1 + 64 i + j (<= last).
-// A chunk (kT * 16 words) with no set bits; its words may be stale scratch
+// A chunk with no set bits; its words may be stale scratch
 // (an extraction skips chunks of windows that hold no frontier state).
 __device__ __forceinline__ bool chunk_empty(const unsigned long long* bsum, uint64_t nbs, uint64_t count,
                                             uint64_t w) {
-    const uint64_t k = w / (kT * 16);
+    const uint64_t k = w / kChunkWords;
     return (k + 1 < nbs ? bsum[k + 1] : count) == bsum[k];
 }
 
@@ -623,7 +641,7 @@ struct SegmentEncoder {
         if (totals) cudaFree(totals);
     }
 
-    static uint64_t chunks(uint64_t n) { return ((n + 63) / 64 + kT * 16 - 1) / (kT * 16); }
+    static uint64_t chunks(uint64_t n) { return ((n + 63) / 64 + kChunkWords - 1) / kChunkWords; }
     static uint32_t max_blocks(uint64_t n) { return uint32_t((n + kBlock - 1) / kBlock); }
 
     int reserve_totals(uint32_t slots, cudaStream_t s) {
@@ -686,7 +704,7 @@ struct SegmentEncoder {
             k_part_bytes<<<part_grid(n), kT, 0, s>>>(idx, t, blocks, refs, cap_refs, psum);
             launches += 2;
         }
-        k_layout<<<1, kScanT, 0, s>>>(t, blocks, psum, cap_refs, with_ops ? 1 : 0, first ? 1 : 0, first_off);
+        k_layout<<<1, kScanT, 0, s>>>(t, blocks, refs, psum, cap_refs, with_ops ? 1 : 0, first ? 1 : 0, first_off);
         launches++;
         CD_CUDA(cudaGetLastError());
         return PSB_OK;
@@ -742,7 +760,7 @@ __device__ __forceinline__ uint64_t every_fourth_bit(uint64_t x) {
 // Frontier bitmap of a two-bit array segment: states whose code is `code`
 // (InMemoryTwoBitBFS.cpp:6-20 layout: bit 2i = code / 2, bit 2i+1 = code % 2).
 // Out word j covers states first + 64 j .. + 63, i.e. code words
-// 2 (first/64 + j) + {0, 1}.  One CTA per chunk of kT * 16 out words, whose
+// 2 (first/64 + j) + {0, 1}.  One CTA per chunk of kChunkWords out words, whose
 // popcount goes to sums[chunk] (the encoder's chunk sums); codes past the
 // last state are 0 and never match.
 // With active-window flags (one byte per 2^wb states, a superset of the
@@ -752,7 +770,7 @@ __device__ __forceinline__ bool chunk_flagged(const uint8_t* flags, int wb, uint
                                               uint64_t n_out, uint64_t base) {
     if (!flags) return true;
     const uint64_t s0 = first + base * 64;
-    const uint64_t end_out = base + kT * 16 < n_out ? base + kT * 16 : n_out;
+    const uint64_t end_out = base + kChunkWords < n_out ? base + kChunkWords : n_out;
     const uint64_t s1 = first + end_out * 64 - 1;
     const uint64_t w0 = s0 >> wb, w1 = (s1 >> wb) < n_windows ? (s1 >> wb) : n_windows - 1;
     int any = 0;
@@ -766,14 +784,14 @@ __global__ void __launch_bounds__(kT) k_frontier_two_bit(const uint64_t* __restr
                                                           const uint8_t* __restrict__ flags, int wb,
                                                           uint64_t n_windows) {
     const uint64_t hi_sel = (code & 2) ? 0 : ~uint64_t(0), lo_sel = (code & 1) ? 0 : ~uint64_t(0);
-    const uint64_t base = uint64_t(blockIdx.x) * kT * 16;
+    const uint64_t base = uint64_t(blockIdx.x) * kChunkWords;
     if (!chunk_flagged(flags, wb, n_windows, first, n_out, base)) {
         if (threadIdx.x == 0) sums[blockIdx.x] = 0;
         return;
     }
     uint32_t c = 0;
-#pragma unroll 4
-    for (int k = 0; k < 16; ++k) {
+#pragma unroll
+    for (int k = 0; k < kCW; ++k) {
         const uint64_t j = base + uint64_t(k) * kT + threadIdx.x;
         if (j < n_out) {
             const uint64_t w = 2 * (first / 64 + j);
@@ -796,9 +814,9 @@ __global__ void __launch_bounds__(kT) k_frontier_nibbles(const uint64_t* __restr
                                                           const uint64_t* __restrict__ excl, uint64_t first,
                                                           uint64_t n_out, uint64_t* __restrict__ out,
                                                           unsigned long long* __restrict__ sums) {
-    const uint64_t base = uint64_t(blockIdx.x) * kT * 16;
+    const uint64_t base = uint64_t(blockIdx.x) * kChunkWords;
     uint32_t c = 0;
-    for (int k = 0; k < 16; ++k) {
+    for (int k = 0; k < kCW; ++k) {
         const uint64_t j = base + uint64_t(k) * kT + threadIdx.x;
         if (j < n_out) {
             const uint64_t w = 4 * (first / 64 + j);
@@ -816,7 +834,7 @@ __global__ void __launch_bounds__(kT) k_frontier_nibbles(const uint64_t* __restr
     chunk_total(c, sums + blockIdx.x);
 }
 
-unsigned chunks_of(uint64_t n_out) { return unsigned((n_out + kT * 16 - 1) / (kT * 16)); }
+unsigned chunks_of(uint64_t n_out) { return unsigned((n_out + kChunkWords - 1) / kChunkWords); }
 
 int frontier_bits_two_bit(const uint64_t* codes, uint64_t first_state, uint64_t n_states, uint32_t code,
                           uint64_t* out, unsigned long long* sums, const uint8_t* flags, int window_bits,
