@@ -255,6 +255,18 @@ __global__ void __launch_bounds__(kThreads) fold_two_bit_flagged(ulonglong2* __r
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, (unsigned long long)c);
 }
 
+// Start of a search on cleared arrays: sets up to three words and one window flag.
+struct SearchStart {
+    uint64_t* word[3];
+    uint64_t value[3];
+    uint8_t* flag;
+};
+__global__ void search_start(SearchStart a) {
+    for (int i = 0; i < 3; ++i)
+        if (a.word[i]) *a.word[i] |= a.value[i];
+    if (a.flag) *a.flag = 1;
+}
+
 }  // namespace psb
 
 namespace {
@@ -790,6 +802,56 @@ int psb::scratch_pool(cudaMemPool_t* pool) {
 
 namespace {
 
+// What a session needs besides device memory: a stream, timing events and a
+// pinned word block.  Making and destroying them took longer than a small
+// search (cudaFreeHost alone up to milliseconds, it waits for the device), so
+// up to kSessionCache sets per device are kept for the next sessions;
+// psb_release_cached_memory frees them.
+struct SessionRes {
+    int device = -1;
+    cudaStream_t stream = nullptr;
+    cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    unsigned long long* h_stats = nullptr;
+    ~SessionRes() {
+        if (h_stats) cudaFreeHost(h_stats);
+        for (auto& e : ev) if (e) cudaEventDestroy(e);
+        if (stream) cudaStreamDestroy(stream);
+    }
+};
+constexpr size_t kSessionCache = 8;
+std::mutex g_session_mu;
+std::vector<SessionRes*> g_session_cache[kMaxPoolDevices];
+
+int session_acquire(int device, SessionRes** out) {
+    {
+        std::lock_guard<std::mutex> lock(g_session_mu);
+        if (device >= 0 && device < kMaxPoolDevices && !g_session_cache[device].empty()) {
+            *out = g_session_cache[device].back();
+            g_session_cache[device].pop_back();
+            return PSB_OK;
+        }
+    }
+    std::unique_ptr<SessionRes> R(new (std::nothrow) SessionRes());
+    if (!R) return fail(PSB_ERR_NOMEM, "session resources");
+    R->device = device;
+    PSB_CUDA(cudaStreamCreateWithFlags(&R->stream, cudaStreamNonBlocking));
+    PSB_CUDA(cudaMallocHost(&R->h_stats, 8 * sizeof(unsigned long long)));
+    for (auto& e : R->ev) PSB_CUDA(cudaEventCreate(&e));
+    *out = R.release();
+    return PSB_OK;
+}
+
+void session_return(SessionRes* R) {
+    {
+        std::lock_guard<std::mutex> lock(g_session_mu);
+        if (R->device >= 0 && R->device < kMaxPoolDevices && g_session_cache[R->device].size() < kSessionCache) {
+            g_session_cache[R->device].push_back(R);
+            return;
+        }
+    }
+    delete R;
+}
+
 // Frontier spill resources: the segment encoder (its device scratch), one
 // segment's extracted bitmap, an arena holding one depth's encoded segments
 // back to back, a copy stream and two pinned host slots.  A depth is encoded
@@ -889,7 +951,6 @@ struct psb_bfs_session {
     psb_puzzle p;
     int algo = 0, mode = 0, device = -1, window_bits = 0;
     cudaStream_t stream = nullptr;
-    bool own_stream = false;
     uint64_t* arr[4] = {nullptr, nullptr, nullptr, nullptr};
     uint64_t words[4] = {0, 0, 0, 0};  // padded sizes
     int n_arr = 0;
@@ -902,7 +963,8 @@ struct psb_bfs_session {
     unsigned long long* h_stats = nullptr;
     uint8_t* wflags[3] = {nullptr, nullptr, nullptr};  // active-window flags (1 byte per window), three levels
     uint64_t n_windows = 0;
-    cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    SessionRes* res = nullptr;
+    cudaEvent_t* ev = nullptr;  // res->ev
     uint64_t bytes = 0;
     cudaMemPool_t pool = nullptr;
     SpillRes* spill = nullptr;  // frontier spill resources, taken from the device's cache on first use
@@ -920,9 +982,12 @@ struct psb_bfs_session {
         if (d_stats) cudaFreeAsync(d_stats, stream);
         for (auto* f : wflags) if (f) cudaFreeAsync(f, stream);
         if (spill) spill_return(spill);
-        if (h_stats) cudaFreeHost(h_stats);
-        for (auto& e : ev) if (e) cudaEventDestroy(e);
-        if (own_stream && stream) cudaStreamDestroy(stream);
+        if (res) {
+            // The next session's work follows this one's on the cached
+            // stream; on a caller's stream it would not.
+            if (stream != res->stream) cudaStreamSynchronize(stream);
+            session_return(res);
+        }
     }
 };
 
@@ -1220,15 +1285,16 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
         S->spill->reset();
     }
     if (S->device >= 0) PSB_CUDA(cudaSetDevice(S->device));
-    for (int i = 0; i < S->n_arr; i++) PSB_CUDA(cudaMemsetAsync(S->arr[i], 0, S->words[i] * 8, s));
-    if (S->visited) PSB_CUDA(cudaMemsetAsync(S->visited, 0, S->words[0] * 8, s));
-    if (S->far && far_marks != PSB_FAR_NONE) PSB_CUDA(cudaMemsetAsync(S->far, 0, S->far_words * 8, s));
-    PSB_CUDA(cudaEventRecord(S->ev[0], s));
+    const bool timed = stats || (opts && opts->level_ms);  // somebody reads the device times
     const int direction = opts ? opts->direction : PSB_DIR_AUTO;
     const double bu_ratio = (opts && opts->bottom_up_ratio > 0) ? double(opts->bottom_up_ratio) : kBottomUpRatio;
     // Three-bit needs its visited array; classic (closed) and two-bit (codes) carry the information.
     const bool can_bu = S->bottom_up && direction != PSB_DIR_TOP_DOWN &&
                         (S->algo != PSB_THREE_BIT || S->visited != nullptr);
+    for (int i = 0; i < S->n_arr; i++) PSB_CUDA(cudaMemsetAsync(S->arr[i], 0, S->words[i] * 8, s));
+    if (S->visited) PSB_CUDA(cudaMemsetAsync(S->visited, 0, S->words[0] * 8, s));
+    if (S->far && far_marks != PSB_FAR_NONE) PSB_CUDA(cudaMemsetAsync(S->far, 0, S->far_words * 8, s));
+    if (timed) PSB_CUDA(cudaEventRecord(S->ev[0], s));
 
     const uint64_t W1 = words_for(N), W2 = words_for(2 * N), W4 = (N + 15) / 16;
     const unsigned grid = unsigned((N + (uint64_t(1) << S->window_bits) - 1) >> S->window_bits);
@@ -1258,16 +1324,21 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
     uint64_t *fcur = S->arr[0], *fnext = S->arr[1], *cex = S->arr[2], *nex = S->arr[3];  // frontier
     uint32_t cur_code = 2;
 
+    psb::SearchStart start{};
+    auto start_bit = [&](int i, uint64_t* words, uint64_t bit) {
+        start.word[i] = words + (bit >> 6);
+        start.value[i] = uint64_t(1) << (bit & 63);
+    };
     switch (S->algo) {
     case PSB_THREE_BIT:
-        if (int rc = set_bit(cur, initial, s)) return rc;
-        if (S->visited) if (int rc = set_bit(S->visited, initial, s)) return rc;
+        start_bit(0, cur, initial);
+        if (S->visited) start_bit(1, S->visited, initial);
         break;
     case PSB_CLASSIC:
-        if (int rc = set_bit(open, initial, s)) return rc;
-        if (int rc = set_bit(closed, initial, s)) return rc;
+        start_bit(0, open, initial);
+        start_bit(1, closed, initial);
         break;
-    case PSB_TWO_BIT: if (int rc = set_bit(codes, 2 * initial, s)) return rc; break;  // code CUR = 2: bit 2i
+    case PSB_TWO_BIT: start_bit(0, codes, 2 * initial); break;  // code CUR = 2: bit 2i
     default: break;
     }
 
@@ -1284,11 +1355,10 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
     const uint64_t sparse_limit = N / 64;
     if (S->algo != PSB_FRONTIER) {
         // Level 0 sweeps only the window of the initial state.
-        static thread_local uint8_t one;
-        one = 1;
         PSB_CUDA(cudaMemsetAsync(S->wflags[0], 0, S->n_windows, s));
-        PSB_CUDA(cudaMemcpyAsync(S->wflags[0] + (initial >> S->window_bits), &one, 1, cudaMemcpyHostToDevice, s));
-        PSB_CUDA(cudaStreamSynchronize(s));
+        start.flag = S->wflags[0] + (initial >> S->window_bits);
+        psb::search_start<<<1, 1, 0, s>>>(start);
+        PSB_CUDA(cudaGetLastError());
         flags_valid = 0;
         flags_old = -2;  // depth -1 is empty
     }
@@ -1344,7 +1414,7 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
         if (produce) PSB_CUDA(cudaMemsetAsync(S->wflags[flags_next], 0, S->n_windows, s));
         a.wflag_cur = flags_valid >= 0 ? S->wflags[flags_valid] : nullptr;
         a.wflag_next = produce ? S->wflags[flags_next] : nullptr;
-        PSB_CUDA(cudaEventRecord(S->ev[1], s));
+        if (timed) PSB_CUDA(cudaEventRecord(S->ev[1], s));
         uint64_t count = 0;
         if (bu) {
             a.wflag_cur = nullptr;
@@ -1382,7 +1452,7 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
             a.far = nullptr;
             launches++;
         }
-        PSB_CUDA(cudaEventRecord(S->ev[2], s));
+        if (timed) PSB_CUDA(cudaEventRecord(S->ev[2], s));
         const bool bu_three = bu && S->algo == PSB_THREE_BIT;
         if (bu_three) {
             // The bottom-up flush already ORed the found states into `visited`,
@@ -1436,14 +1506,16 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
             PSB_CUDA(cudaGetLastError());
             others++;
         }
-        PSB_CUDA(cudaEventRecord(S->ev[3], s));
+        if (timed) PSB_CUDA(cudaEventRecord(S->ev[3], s));
         if (spill) if (int rc = spill_drain(S->spill, opts, &spilled)) return rc;  // overlaps this level
         PSB_CUDA(cudaMemcpyAsync(S->h_stats, S->d_stats, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
         PSB_CUDA(cudaStreamSynchronize(s));
         if (S->h_stats[3]) return fail(PSB_ERR_DEVICE, "level kernel produced a child index >= IndexesCount()");
         float t_exp = 0, t_fin = 0;
-        PSB_CUDA(cudaEventElapsedTime(&t_exp, S->ev[1], S->ev[2]));
-        PSB_CUDA(cudaEventElapsedTime(&t_fin, S->ev[2], S->ev[3]));
+        if (timed) {
+            PSB_CUDA(cudaEventElapsedTime(&t_exp, S->ev[1], S->ev[2]));
+            PSB_CUDA(cudaEventElapsedTime(&t_fin, S->ev[2], S->ev[3]));
+        }
         expand_ms += t_exp;
         finalize_ms += t_fin;
         expanded += (S->algo == PSB_FRONTIER && first) ? 1 : S->h_stats[0];
@@ -1514,10 +1586,12 @@ done:
         if (int rc = spill_depth(S, opts, spilled_depths, src, &spilled)) return rc;
     }
     if (spill) if (int rc = spill_drain(S->spill, opts, &spilled)) return rc;
-    PSB_CUDA(cudaEventRecord(S->ev[3], s));
-    PSB_CUDA(cudaEventSynchronize(S->ev[3]));
     float total = 0;
-    PSB_CUDA(cudaEventElapsedTime(&total, S->ev[0], S->ev[3]));
+    if (timed) {
+        PSB_CUDA(cudaEventRecord(S->ev[3], s));
+        PSB_CUDA(cudaEventSynchronize(S->ev[3]));
+        PSB_CUDA(cudaEventElapsedTime(&total, S->ev[0], S->ev[3]));
+    }
     if (res.size() > cap) return fail(PSB_ERR_CAPACITY, "more than %u depths", cap);
     std::copy(res.begin(), res.end(), counts);
     *n_depths = uint32_t(res.size());
@@ -1599,11 +1673,10 @@ int psb_bfs_session_create(const psb_puzzle* p, int algo, const psb_bfs_opts* op
         return fail(PSB_ERR_ARG, "window_bits %d out of range", S->window_bits);
     if (((p->n_states + (uint64_t(1) << S->window_bits) - 1) >> S->window_bits) > 0x7FFFFFFFull)
         return fail(PSB_ERR_ARG, "too many windows");
-    if (opts && opts->stream) S->stream = static_cast<cudaStream_t>(opts->stream);
-    else {
-        PSB_CUDA(cudaStreamCreateWithFlags(&S->stream, cudaStreamNonBlocking));
-        S->own_stream = true;
-    }
+    if (int rc = session_acquire(S->device, &S->res)) return rc;
+    S->stream = opts && opts->stream ? static_cast<cudaStream_t>(opts->stream) : S->res->stream;
+    S->ev = S->res->ev;
+    S->h_stats = S->res->h_stats;
     if (int rc = session_pool(S->device, &S->pool)) return rc;
     for (int i = 0; i < S->n_arr; i++)
         if (int rc = S->alloc(reinterpret_cast<void**>(&S->arr[i]), S->words[i] * 8)) return rc;
@@ -1636,8 +1709,6 @@ int psb_bfs_session_create(const psb_puzzle* p, int algo, const psb_bfs_opts* op
     for (auto& f : S->wflags)
         if (int rc = S->alloc(reinterpret_cast<void**>(&f), S->n_windows)) return rc;
     if (int rc = S->alloc(reinterpret_cast<void**>(&S->d_stats), 8 * sizeof(unsigned long long))) return rc;
-    PSB_CUDA(cudaMallocHost(&S->h_stats, 8 * sizeof(unsigned long long)));
-    for (auto& e : S->ev) PSB_CUDA(cudaEventCreate(&e));
     *out = S.release();
     return PSB_OK;
 }
@@ -1669,6 +1740,12 @@ int psb_release_cached_memory(int device) {
         cached.swap(g_spill_cache[device]);
     }
     for (SpillRes* R : cached) delete R;
+    std::vector<SessionRes*> sessions;
+    {
+        std::lock_guard<std::mutex> lock(g_session_mu);
+        sessions.swap(g_session_cache[device]);
+    }
+    for (SessionRes* R : sessions) delete R;
     if (!pool) return PSB_OK;
     PSB_CUDA(cudaDeviceSynchronize());  // frees still queued on streams return first
     PSB_CUDA(cudaMemPoolTrimTo(pool, 0));
