@@ -203,7 +203,7 @@ typedef struct {
 
 typedef struct {
     uint32_t struct_size;     /* sizeof(psb_bfs_stats) */
-    uint32_t levels;          /* level kernels launched */
+    uint32_t levels;          /* BFS levels run */
     uint32_t window_bits;     /* window used */
     uint32_t threads;         /* threads per block of the level kernel */
     double total_ms;          /* device time of the whole search (CUDA events) */
@@ -212,7 +212,7 @@ typedef struct {
     uint64_t expanded;        /* parents expanded */
     uint64_t children;        /* valid children generated */
     uint64_t local_children;  /* children marked in the block's shared-memory window */
-    uint64_t expand_launches; /* level-kernel launches (one per level) */
+    uint64_t expand_launches; /* level-kernel launches (one per level; 1 for a small search run in one launch) */
     uint64_t device_bytes;    /* device memory held by the search */
     uint64_t bottom_up_levels; /* levels that ran bottom-up (their "children" are probes) */
     double spill_ms;          /* host time in the spill: encoding plus handing over (the latter overlaps the

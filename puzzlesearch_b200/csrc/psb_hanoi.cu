@@ -4,6 +4,7 @@
 
 #include "psb_hanoi_words.cuh"
 #include "psb_kernels.cuh"
+#include "psb_small.cuh"
 
 namespace psb {
 
@@ -62,6 +63,7 @@ bool hanoi_kernels(PuzzleKernels* out) {
     out->level_shape[1][kTwoBit] = &launch_hanoi_level<kTwoBit, 1>;
     out->level_shape[2][kThreeBit] = &launch_hanoi_level<kThreeBit, 2>;
     out->level_shape[2][kTwoBit] = &launch_hanoi_level<kTwoBit, 2>;
+    out->small = &launch_small_search<HanoiK>;
     return true;
 }
 

@@ -819,6 +819,7 @@ struct SessionRes {
     }
 };
 constexpr size_t kSessionCache = 8;
+constexpr size_t kSmallOut = psb::kSmallHeader + 2 * psb::kSmallDepths;  // words of a small search's result
 std::mutex g_session_mu;
 std::vector<SessionRes*> g_session_cache[kMaxPoolDevices];
 
@@ -835,7 +836,7 @@ int session_acquire(int device, SessionRes** out) {
     if (!R) return fail(PSB_ERR_NOMEM, "session resources");
     R->device = device;
     PSB_CUDA(cudaStreamCreateWithFlags(&R->stream, cudaStreamNonBlocking));
-    PSB_CUDA(cudaMallocHost(&R->h_stats, 8 * sizeof(unsigned long long)));
+    PSB_CUDA(cudaMallocHost(&R->h_stats, std::max<size_t>(8, kSmallOut) * sizeof(unsigned long long)));
     for (auto& e : R->ev) PSB_CUDA(cudaEventCreate(&e));
     *out = R.release();
     return PSB_OK;
@@ -864,6 +865,12 @@ struct SpillSeg {
     uint32_t depth, segment;
     uint64_t off, bytes, states;
 };
+
+// Searches of up to kSmallChildren children run in one launch, on 16 SMs; larger
+// ones level by level on all of them, a host round trip each.  On B200 (level
+// by level -> one launch): 10-disk Hanoi (6.3 M children) 1.35 -> 1.13 ms, 2x5
+// board (14.5 M) 1.91 -> 1.22 ms, 10 pancakes (32.7 M) 0.63 -> 1.29 ms.
+constexpr uint64_t kSmallChildren = uint64_t(1) << 24;
 
 constexpr uint32_t kSpillBatch = 256;  // segments encoded between two waits
 
@@ -961,6 +968,7 @@ struct psb_bfs_session {
     bool bottom_up = false;       // this search's algorithm and puzzle support bottom-up levels
     unsigned long long* d_stats = nullptr;
     unsigned long long* h_stats = nullptr;
+    unsigned long long* small = nullptr;  // small_search's result (PuzzleKernels::small)
     uint8_t* wflags[3] = {nullptr, nullptr, nullptr};  // active-window flags (1 byte per window), three levels
     uint64_t n_windows = 0;
     SessionRes* res = nullptr;
@@ -981,6 +989,7 @@ struct psb_bfs_session {
         if (far) cudaFreeAsync(far, stream);
         if (d_stats) cudaFreeAsync(d_stats, stream);
         for (auto* f : wflags) if (f) cudaFreeAsync(f, stream);
+        if (small) cudaFreeAsync(small, stream);
         if (spill) spill_return(spill);
         if (res) {
             // The next session's work follows this one's on the cached
@@ -1263,6 +1272,36 @@ int spill_depth(psb_bfs_session* S, const psb_bfs_opts* o, uint32_t depth, const
     return PSB_OK;
 }
 
+// Runs a whole two-bit search in one launch (psb_small.cuh): S->h_stats holds
+// its result afterwards.  *done false: too deep for it, or no cluster of that
+// size here; nothing has happened to the session that a search does not reset.
+int small_search(psb_bfs_session* S, uint64_t initial, uint32_t max_depth, int direction, double ratio, bool can_bu,
+                 bool codes, bool* done) {
+    psb::SmallArgs a{};
+    a.n_states = S->p.n_states;
+    a.initial = initial;
+    a.codes = codes ? S->arr[0] : nullptr;
+    a.code_words = words_for(2 * S->p.n_states);
+    a.out = S->small;
+    a.ratio = ratio;
+    a.pz = S->p.pz;
+    a.max_levels = max_depth ? max_depth + 1 : 0xFFFFFFFFu;
+    a.bits = 10;
+    while (S->p.n_states > uint64_t(psb::kSmallBlocks) << a.bits) a.bits++;
+    a.direction = direction;
+    a.can_bu = can_bu ? 1 : 0;
+    *done = false;
+    if (S->p.k.small(a, S->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return PSB_OK;
+    }
+    PSB_CUDA(cudaMemcpyAsync(S->h_stats, a.out, kSmallOut * 8, cudaMemcpyDeviceToHost, S->stream));
+    PSB_CUDA(cudaStreamSynchronize(S->stream));
+    if (S->h_stats[0] == 1) return fail(PSB_ERR_DEVICE, "level kernel produced a child index >= IndexesCount()");
+    *done = S->h_stats[0] == 0;
+    return PSB_OK;
+}
+
 int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, uint64_t* counts, uint32_t cap,
                 uint32_t* n_depths, psb_bfs_stats* stats) {
     const psb_puzzle& P = S->p;
@@ -1291,10 +1330,19 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
     // Three-bit needs its visited array; classic (closed) and two-bit (codes) carry the information.
     const bool can_bu = S->bottom_up && direction != PSB_DIR_TOP_DOWN &&
                         (S->algo != PSB_THREE_BIT || S->visited != nullptr);
-    for (int i = 0; i < S->n_arr; i++) PSB_CUDA(cudaMemsetAsync(S->arr[i], 0, S->words[i] * 8, s));
-    if (S->visited) PSB_CUDA(cudaMemsetAsync(S->visited, 0, S->words[0] * 8, s));
-    if (S->far && far_marks != PSB_FAR_NONE) PSB_CUDA(cudaMemsetAsync(S->far, 0, S->far_words * 8, s));
-    if (timed) PSB_CUDA(cudaEventRecord(S->ev[0], s));
+    // A small two-bit search with nothing to hand over between its levels
+    // runs in one launch.
+    bool whole = false;
+    if (S->small && !spill && !restored && !(opts && (opts->level_ms || opts->far_marks || opts->threads))) {
+        if (timed) PSB_CUDA(cudaEventRecord(S->ev[0], s));
+        if (int rc = small_search(S, initial, max_depth, direction, bu_ratio, can_bu, opts && opts->final_words, &whole)) return rc;
+    }
+    if (!whole) {
+        for (int i = 0; i < S->n_arr; i++) PSB_CUDA(cudaMemsetAsync(S->arr[i], 0, S->words[i] * 8, s));
+        if (S->visited) PSB_CUDA(cudaMemsetAsync(S->visited, 0, S->words[0] * 8, s));
+        if (S->far && far_marks != PSB_FAR_NONE) PSB_CUDA(cudaMemsetAsync(S->far, 0, S->far_words * 8, s));
+        if (timed) PSB_CUDA(cudaEventRecord(S->ev[0], s));
+    }
 
     const uint64_t W1 = words_for(N), W2 = words_for(2 * N), W4 = (N + 15) / 16;
     const unsigned grid = unsigned((N + (uint64_t(1) << S->window_bits) - 1) >> S->window_bits);
@@ -1353,7 +1401,7 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
     int flags_old = -1;            // windows of the previous depth: -1 unknown, -2 none
     uint64_t estimate = 1;         // last known frontier size
     const uint64_t sparse_limit = N / 64;
-    if (S->algo != PSB_FRONTIER) {
+    if (S->algo != PSB_FRONTIER && !whole) {
         // Level 0 sweeps only the window of the initial state.
         PSB_CUDA(cudaMemsetAsync(S->wflags[0], 0, S->n_windows, s));
         start.flag = S->wflags[0] + (initial >> S->window_bits);
@@ -1371,7 +1419,22 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
     const bool want_final = opts && opts->final_words;
     bool first = true;
     uint32_t iteration = 0;
-    for (;;) {
+    uint64_t levels = 0;  // BFS levels run
+    if (whole) {
+        const unsigned long long* h = S->h_stats;
+        levels = h[1];
+        launches = 1;
+        bu_levels = h[2];
+        expanded = h[3];
+        children = h[4];
+        local = h[5];
+        for (uint64_t l = 0; l < levels; l++) {
+            const uint64_t count = h[psb::kSmallHeader + 2 * l];
+            if (opts && opts->level_children && l < cap) opts->level_children[l] = h[psb::kSmallHeader + 2 * l + 1];
+            if (count) res.push_back(count);
+        }
+    }
+    while (!whole) {
         if (max_depth && res.size() >= size_t(max_depth) + 1) break;
         if (spill) {  // the states at depth `iteration`, before its level changes the arrays
             SpillSource src;
@@ -1617,11 +1680,11 @@ done:
         PSB_CUDA(cudaStreamSynchronize(s));
     }
     if (stats && stats->struct_size >= sizeof(psb_bfs_stats)) {
-        stats->levels = uint32_t(launches);
+        stats->levels = uint32_t(whole ? levels : launches);
         stats->window_bits = uint32_t(S->window_bits);
         stats->threads = uint32_t(variant ? psb::variant_threads(variant) : psb::level_threads(S->mode));
         stats->total_ms = total;
-        stats->expand_ms = expand_ms;
+        stats->expand_ms = whole ? total : expand_ms;
         stats->finalize_ms = finalize_ms;
         stats->expanded = expanded;
         stats->children = children;
@@ -1709,6 +1772,10 @@ int psb_bfs_session_create(const psb_puzzle* p, int algo, const psb_bfs_opts* op
     for (auto& f : S->wflags)
         if (int rc = S->alloc(reinterpret_cast<void**>(&f), S->n_windows)) return rc;
     if (int rc = S->alloc(reinterpret_cast<void**>(&S->d_stats), 8 * sizeof(unsigned long long))) return rc;
+    if (algo == PSB_TWO_BIT && p->k.small && S->own_windows &&
+        p->n_states <= kSmallChildren / uint64_t(p->branching)) {
+        if (int rc = S->alloc(reinterpret_cast<void**>(&S->small), kSmallOut * 8)) return rc;
+    }
     *out = S.release();
     return PSB_OK;
 }

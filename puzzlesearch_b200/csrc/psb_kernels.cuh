@@ -1234,6 +1234,27 @@ __global__ void __launch_bounds__(kThreads) segment_expand_kernel(SegExpandArgs 
 }
 
 // ---------------------------------------------------------------------------
+// Whole two-bit searches of small puzzles in one launch (psb_small.cuh).
+// ---------------------------------------------------------------------------
+constexpr int kSmallBlocks = 16, kSmallThreads = 512;
+constexpr uint32_t kSmallDepths = 1024;  // deeper searches run level by level
+constexpr int kSmallHeader = 6;          // words before the depths' (count, children) pairs
+constexpr int kSmallBottomUp = 2;        // SmallArgs::direction (PSB_DIR_BOTTOM_UP); 0: automatic
+struct SmallArgs {
+    uint64_t n_states, initial;
+    uint64_t* codes;          // final two-bit codes (NULL: not wanted)
+    uint64_t code_words;
+    unsigned long long* out;  // status (1: bad child, 2: too deep), levels, bottom-up levels, expanded, children,
+                              // local children, then each level's count and children
+    double ratio;             // bottom-up below ratio x frontier unvisited states
+    PuzzleArgs pz;
+    uint32_t max_levels;
+    int bits;                 // log2 states per block: kSmallBlocks << bits >= n_states
+    int direction, can_bu;
+};
+using SmallLaunch = cudaError_t (*)(const SmallArgs&, cudaStream_t);
+
+// ---------------------------------------------------------------------------
 // Launch helpers and per-puzzle dispatch tables.
 // ---------------------------------------------------------------------------
 using LevelLaunch = cudaError_t (*)(const LevelArgs&, unsigned grid, size_t smem, cudaStream_t);
@@ -1250,6 +1271,7 @@ struct PuzzleKernels {
     SeedLaunch seed;
     ExpandLaunch expand;
     SegExpandLaunch segment_expand;
+    SmallLaunch small;  // NULL: no whole-search kernel for this puzzle
     int branching;
 };
 
@@ -1311,6 +1333,7 @@ PuzzleKernels make_kernels() {
     k.seed = &launch_seed<PZ>;
     k.expand = &launch_expand<PZ>;
     k.segment_expand = &launch_segment_expand<PZ>;
+    k.small = nullptr;
     k.branching = PZ::kBranch;
     return k;
 }

@@ -2,6 +2,7 @@
 // instantiation per size: sizes 2..16 (PancakeSimple.cpp:26).
 #include "psb_kernels.cuh"
 #include "psb_pancake_windows.cuh"
+#include "psb_small.cuh"
 
 namespace psb {
 
@@ -17,6 +18,8 @@ PuzzleKernels pancake_table() {
         k.level_shape[1][kTwoBit] = &launch_pancake_level<N, kTwoBit, 1>;
         k.level_shape[2][kThreeBit] = &launch_pancake_level<N, kThreeBit, 2>;
         k.level_shape[2][kTwoBit] = &launch_pancake_level<N, kTwoBit, 2>;
+    } else {
+        k.small = &launch_small_search<PancakeK<N>>;
     }
     return k;
 }

@@ -4,12 +4,22 @@
 // SlidingTilePuzzleOptimized.cpp:293-307); the width is a runtime argument,
 // so 2x3 or 3x4 boards run too.
 #include "psb_kernels.cuh"
+#include "psb_small.cuh"
 
 namespace psb {
 
+namespace {
+template <int N>
+PuzzleKernels table() {
+    PuzzleKernels k = make_kernels<SlidingOptK<N>>();
+    if constexpr (N <= 10) k.small = &launch_small_search<SlidingOptK<N>>;
+    return k;
+}
+}  // namespace
+
 bool sliding_opt_kernels(int cells, PuzzleKernels* out) {
     switch (cells) {
-#define PSB_CASE(N) case N: *out = make_kernels<SlidingOptK<N>>(); return true;
+#define PSB_CASE(N) case N: *out = table<N>(); return true;
         PSB_CASE(4) PSB_CASE(6) PSB_CASE(8) PSB_CASE(9) PSB_CASE(10) PSB_CASE(12) PSB_CASE(14) PSB_CASE(15)
         PSB_CASE(16)
 #undef PSB_CASE

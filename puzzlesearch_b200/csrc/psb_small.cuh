@@ -1,0 +1,210 @@
+// psb_small.cuh -- a whole two-bit search of a small puzzle in one launch.
+//
+// A level of a small search (3x3 board: at most 24,047 states) is a few
+// microseconds of work, and launching it, clearing its counters, reading them
+// back and waiting cost 28 us on the host, level after level.  Here one
+// cluster of 16 blocks runs all levels.  Each block owns a sixteenth of the
+// states as three bitmaps in its shared memory (visited, frontier, marks);
+// children are marked in their owner's shared memory, the cluster's hardware
+// barrier separates the levels, and every block takes psb_bfs's decisions
+// (direction, end of the search) from counts the blocks exchange.  Global
+// memory sees the final codes and the counts only.  B200, whole calls: 3x3 board
+// 950 -> 232 us (32 levels, 6 us each), 8 pancakes 342 -> 96 us, 8-disk Hanoi
+// 922 -> 306 us.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "psb_kernels.cuh"
+
+namespace psb {
+
+// One block's share of a level's counters, written into every block.
+struct SmallCounts {
+    unsigned long long next, children, local, bad;
+};
+
+// Children of the frontier: marked in their owner's bitmap.
+struct SmallMarker {
+    uint32_t* marks;  // this block's
+    uint64_t n_states;
+    uint32_t rank;
+    int bits;
+    uint32_t children = 0, local = 0, bad = 0;
+    __device__ __forceinline__ void operator()(uint64_t c, uint32_t) {
+        if (c >= n_states) { bad = 1; return; }  // never expected: keeps a bad index off the memory system
+        ++children;
+        const uint32_t owner = uint32_t(c >> bits), o = uint32_t(c) & ((1u << bits) - 1u);
+        uint32_t* word = marks + (o >> 5);
+        if (owner == rank) ++local;
+        else word = cooperative_groups::this_cluster().map_shared_rank(word, owner);
+        atomicOr(word, 1u << (o & 31u));
+    }
+};
+
+// Neighbours of an unvisited state: is one of them in the frontier?
+struct SmallProbe {
+    uint32_t* front;  // this block's
+    uint64_t n_states;
+    uint32_t rank;
+    int bits;
+    uint32_t probes = 0, hit = 0, bad = 0;
+    __device__ __forceinline__ void operator()(uint64_t c, uint32_t) {
+        if (c >= n_states) { bad = 1; return; }
+        ++probes;
+        const uint32_t owner = uint32_t(c >> bits), o = uint32_t(c) & ((1u << bits) - 1u);
+        uint32_t* word = front + (o >> 5);
+        if (owner != rank) word = cooperative_groups::this_cluster().map_shared_rank(word, owner);
+        hit |= (*word >> (o & 31u)) & 1u;
+    }
+};
+
+template <class PZ>
+__global__ void __launch_bounds__(kSmallThreads, 1) small_search_kernel(SmallArgs a) {
+    extern __shared__ __align__(16) uint32_t small_mem[];
+    __shared__ SmallCounts parts[2][kSmallBlocks];  // of levels l and l + 1
+    __shared__ unsigned long long own[4];
+    constexpr int T = kSmallThreads;
+    auto cluster = cooperative_groups::this_cluster();
+    const uint32_t rank = cluster.block_rank(), tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t units = 1u << (a.bits - 5);  // 32 states each
+    uint32_t *visited = small_mem, *front = visited + units, *marks = front + units;
+    uint16_t* list = reinterpret_cast<uint16_t*>(marks + units) + warp * 1024;
+    const uint64_t n = a.n_states, base = uint64_t(rank) << a.bits;
+
+    for (uint32_t u = tid; u < 3 * units; u += T) small_mem[u] = 0;
+    if (tid < 4) own[tid] = 0;
+    __syncthreads();
+    if (tid == 0 && (a.initial >> a.bits) == rank) {
+        const uint32_t o = uint32_t(a.initial - base);
+        visited[o >> 5] = front[o >> 5] = 1u << (o & 31u);
+    }
+    cluster.sync();
+
+    uint32_t level = 0, status = 0, bu_levels = 0;
+    uint64_t seen = 0, frontier = 1, expanded = 0, children = 0, local = 0;
+    while (level < a.max_levels) {
+        if (level >= kSmallDepths) { status = 2; break; }
+        const uint64_t unvisited = n - (seen + frontier < n ? seen + frontier : n);
+        const bool bu = a.can_bu && (a.direction == kSmallBottomUp ||
+                                     (a.direction == 0 && frontier >= n / 64 && double(unvisited) < a.ratio * double(frontier)));
+        SmallMarker mark{marks, n, rank, a.bits};
+        SmallProbe probe{front, n, rank, a.bits};
+        // A warp lists the states of 32 words and expands them 32 at a time.
+        for (uint32_t u0 = warp * 32; u0 < units; u0 += T) {
+            const uint32_t u = u0 + lane;
+            uint32_t m = bu ? ~visited[u] : front[u];
+            if (bu) {  // states below n_states only
+                const uint64_t first = base + 32ull * u;
+                if (first + 32 > n) m &= first < n ? (1u << uint32_t(n - first)) - 1u : 0u;
+            }
+            uint32_t incl = __popc(m);
+            const uint32_t c = incl;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= uint32_t(o)) incl += y;
+            }
+            const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            uint32_t at = incl - c;
+            while (m) {
+                list[at++] = uint16_t(lane * 32 + __ffs(m) - 1);
+                m &= m - 1;
+            }
+            __syncwarp();
+            for (uint32_t e = lane; e < total; e += 32) {
+                const uint32_t o = u0 * 32 + list[e];
+                if (bu) {
+                    probe.hit = 0;
+                    PZ::template expand<false>(base + o, 0u, a.pz, probe);
+                    if (probe.hit) atomicOr(&marks[o >> 5], 1u << (o & 31u));
+                } else {
+                    PZ::template expand<false>(base + o, 0u, a.pz, mark);
+                }
+            }
+            __syncwarp();
+        }
+        cluster.sync();  // every mark is made, every probe has read
+        // The marked states not visited yet are the next frontier.
+        uint32_t found = 0;
+        for (uint32_t u = tid; u < units; u += T) {
+            const uint32_t v = visited[u], f = marks[u] & ~v;
+            if (marks[u]) marks[u] = 0;
+            front[u] = f;
+            if (f) visited[u] = v | f;
+            found += __popc(f);
+        }
+        const uint32_t sum[4] = {found, bu ? probe.probes : mark.children, bu ? 0u : mark.local,
+                                 bu ? probe.bad : mark.bad};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t t = __reduce_add_sync(0xFFFFFFFFu, sum[i]);
+            if (lane == 0 && t) atomicAdd(&own[i], (unsigned long long)t);
+        }
+        __syncthreads();
+        // Into every block: thread i writes block i's copy.
+        if (tid < kSmallBlocks)
+            *cluster.map_shared_rank(&parts[level & 1][rank], tid) = SmallCounts{own[0], own[1], own[2], own[3]};
+        cluster.sync();
+        if (tid < 4) own[tid] = 0;
+        SmallCounts all{0, 0, 0, 0};
+        for (int i = 0; i < kSmallBlocks; ++i) {
+            const SmallCounts& p = parts[level & 1][i];
+            all.next += p.next;
+            all.children += p.children;
+            all.local += bu ? p.next : p.local;
+            all.bad += p.bad;
+        }
+        if (rank == 0 && tid == 0) {
+            a.out[kSmallHeader + 2 * level] = frontier;
+            a.out[kSmallHeader + 2 * level + 1] = all.children;
+        }
+        expanded += bu ? unvisited : frontier;
+        children += all.children;
+        local += all.local;
+        bu_levels += bu ? 1 : 0;
+        if (all.bad) { status = 1; break; }
+        ++level;
+        seen += frontier;
+        frontier = all.next;
+        if (frontier == 0) break;
+    }
+    if (rank == 0 && tid == 0) {
+        const uint64_t head[kSmallHeader] = {status, level, bu_levels, expanded, children, local};
+        for (int i = 0; i < kSmallHeader; ++i) a.out[i] = head[i];
+    }
+    if (a.codes) {
+        // The reference's codes: visited states OLD (1), the last depth's CUR,
+        // 2 at even depths and 3 at odd ones (bit 2i = code / 2, bit 2i + 1 = code % 2).
+        for (uint32_t u = tid; u < units; u += T) {
+            const uint64_t w = (base >> 5) + u;
+            if (w >= a.code_words) break;
+            const uint64_t f = spread_even(front[u]), old = spread_even(visited[u] & ~front[u]);
+            a.codes[w] = f | ((old | ((level & 1) ? f : 0)) << 1);
+        }
+    }
+    cluster.sync();  // no block leaves while others may still reach into it
+}
+
+template <class PZ>
+cudaError_t launch_small_search(const SmallArgs& a, cudaStream_t s) {
+    const size_t smem = 3 * (size_t(1) << a.bits) / 8 + kSmallThreads / 32 * 1024 * 2;
+    cudaError_t e = cudaFuncSetAttribute(small_search_kernel<PZ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(small_search_kernel<PZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kSmallBlocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kSmallBlocks);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, small_search_kernel<PZ>, a);
+}
+
+}  // namespace psb

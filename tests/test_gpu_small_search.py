@@ -1,0 +1,50 @@
+"""Two-bit searches that run whole in one launch, against the oracle and the
+level-by-level path (asked for by window_bits): index spaces from two states
+to the largest that run this way, not multiples of a block's share or of 64,
+all directions, searches stopped part-way, packed indexes and peg symmetry."""
+import pytest
+
+import oracle as O
+import puzzlesearch_b200 as psb
+from _puzzles import make
+
+pytestmark = pytest.mark.gpu
+
+SPECS = ([["pancake", n, 0] for n in (2, 3, 6, 7, 9)] + [["sliding", w, h] for w, h in ((1, 2), (2, 2), (7, 1), (2, 4), (3, 3))]
+         + [["hanoi4", n, s] for n, s in ((1, 0), (2, 1), (5, 0), (8, 1), (9, 0))]
+         + [["sliding_opt", 2, 2], ["sliding_opt", 3, 3], ["hanoi4_opt", 8, 1], ["pancake_opt", 8, 0]])
+
+
+@pytest.mark.parametrize("spec", SPECS, ids=lambda s: f"{s[0]}{s[1]}x{s[2]}")
+def test_counts_and_final_arrays(spec):
+    p = make(spec)
+    n = p.IndexesCount()
+    if spec[0] == "sliding_opt":
+        starts = [O.parse(spec, " ".join(str(i) for i in range(spec[1] * spec[2])))]
+    else:
+        starts = {0, n - 1, n * 5 // 7} if not spec[2] or spec[0] == "sliding" else {0}
+    for start in starts:
+        counts, final = O.bfs(spec, "two_bit", start, final=True)
+        for direction in ("auto", "top_down", "bottom_up"):
+            r = psb.bfs(p, "two_bit", start, final=True, direction=direction)
+            assert r["stats"]["expand_launches"] == 1
+            assert r["counts"] == counts and r["final"] == final, direction
+        for md in {1, 2, len(counts) // 2, len(counts) - 1, len(counts) + 3} - {0}:
+            r = psb.bfs(p, "two_bit", start, final=True, max_depth=md)
+            want = psb.bfs(p, "two_bit", start, final=True, max_depth=md, window_bits=10)
+            assert want["stats"]["expand_launches"] > 1 or len(counts) == 1 or md < 2
+            assert r["counts"] == counts[:md + 1]
+            assert r["final"] == want["final"], md
+
+
+def test_children_and_sessions():
+    """Children per depth without level times; a session's arrays hold no
+    trace of the search before."""
+    p = psb.SlidingTilePuzzleSimple(3, 3)
+    want = psb.bfs(p, "two_bit", 5, direction="top_down", window_bits=10)["stats"]
+    got = psb.bfs(p, "two_bit", 5, direction="top_down")["stats"]
+    assert (got["children"], got["expanded"], got["levels"]) == (want["children"], want["expanded"], want["levels"])
+    s = psb.BfsSession(p, "two_bit")
+    for start in (5, 0, 5, 362879):
+        assert s.run(start)[0] == O.bfs(["sliding", 3, 3], "two_bit", start)[0]
+    s.close()
