@@ -60,7 +60,7 @@ struct Shape {
     static constexpr int threads = V == 1 ? 512 : V == 2 ? 128 : 256;
     static constexpr int min_blocks = BU ? 4
                                     : MODE == kTwoBit ? (V == 1 ? 1 : V == 2 ? 5 : 4)
-                                    : MODE == kFrontier ? 2
+                                    : MODE == kFrontier ? 3
                                     : (V == 2 ? 2 : 1);
 };
 constexpr int kShapeVariants = 3;
@@ -114,10 +114,6 @@ struct PancakeK {
     template <bool kOpBits, class E>
     __device__ __forceinline__ static void expand(uint64_t i, uint32_t ob, const PuzzleArgs&, E& e) {
         Pancake<N>::template expand<kOpBits>(i, ob, e);
-    }
-    template <int F, class E>
-    __device__ __forceinline__ static void expand_from(uint64_t i, const PuzzleArgs&, E& e) {
-        Pancake<N>::template expand_range<false>(i, 0u, F, N - 1, e);
     }
     template <class E>
     __device__ __forceinline__ static void probe_range(uint64_t i, int first, int last, const PuzzleArgs&, E& e) {
@@ -347,7 +343,7 @@ __host__ __device__ constexpr size_t mark_bytes(int mode, size_t window_states) 
 
 // Warp chunk: 32 lanes x one unit each (64 states; 32 for two-bit codes).
 __host__ __device__ constexpr uint32_t states_per_unit(int mode) { return mode == kTwoBit ? 32 : 64; }
-__host__ __device__ constexpr size_t list_entry_bytes(int mode) { return mode == kFrontier ? 4 : 2; }
+__host__ __device__ constexpr size_t list_entry_bytes(int) { return 2; }  // 11 bits of offset, 4 operator bits above
 constexpr size_t kWarpScratch = 256;  // per warp: the chunk's two unranking prefixes (kChunkPrefix)
 
 // Dynamic shared memory of a level_window pass: window marks, then one list
@@ -664,7 +660,8 @@ __device__ __forceinline__ void level_window(const LevelArgs& a, uint64_t window
     const uint32_t chunks = (units + 31) / 32;
     const uint32_t mbytes = uint32_t(mark_bytes(MODE, W));
     uint32_t* smarks = reinterpret_cast<uint32_t*>(smem64);
-    using Entry = typename std::conditional<MODE == kFrontier, uint32_t, uint16_t>::type;
+    using Entry = uint16_t;
+    static_assert(kChunk <= 2048, "a chunk's offsets take 11 bits");
     Entry* wlist = reinterpret_cast<Entry*>(reinterpret_cast<char*>(smem64) + mbytes) + size_t(warp) * kChunk;
     // Unranking prefixes of the chunk's (at most two) blocks of PZ::kBlock indexes.
     constexpr bool kPrefixed = PZ::kChunkPrefix && MODE != kFrontier;
@@ -700,6 +697,14 @@ __device__ __forceinline__ void level_window(const LevelArgs& a, uint64_t window
     };
     uint32_t probes = 0, hits = 0, pbad = 0;  // bottom-up counters
     uint32_t mult = 0;                         // sum of the frontier states' class sizes (sym_mult)
+    // Puzzles without chunk prefixes expand whole waves only: the states of a
+    // chunk past the last 32 wait in registers, one per lane, for the next
+    // chunk's (a 1024-state chunk of the 3x4 board lists 47 at its densest
+    // level).  The prefixed expansion is tied to its chunk, and pancakes lost
+    // more by the carried state than they gained by full waves.
+    constexpr bool kCarry = !BU && !kPrefixed;
+    static_assert(kCarry || BU || MODE != kFrontier, "frontier search carries");
+    uint32_t carry = 0, carried = 0;
 
     // Each warp takes chunks on its own (its first chunk is its warp index,
     // later ones come from a shared counter): lane l sweeps unit 32*chunk + l,
@@ -859,7 +864,7 @@ __device__ __forceinline__ void level_window(const LevelArgs& a, uint64_t window
             if constexpr (MODE == kFrontier) {
                 const uint64_t word = j < 16 ? cw[0 % kWPU] : j < 32 ? cw[1 % kWPU] : j < 48 ? cw[2 % kWPU] : cw[3 % kWPU];
                 const uint32_t bits = uint32_t(word >> (4 * (j & 15))) & 15u;
-                return Entry((ub + j) | (bits << 16));
+                return Entry((ub + j) | (bits << 11));
             } else {
                 return Entry(ub + j);
             }
@@ -871,7 +876,8 @@ __device__ __forceinline__ void level_window(const LevelArgs& a, uint64_t window
             if (lane >= o) incl += y;
         }
         const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        if (total) {
+        const bool last = kCarry && nch >= chunks;  // the warp's last chunk: nothing is carried on
+        if (total || (last && carried)) {
             uint32_t off = incl - cnt;
             while (pmask) {
                 const uint32_t j = __ffsll((long long)pmask) - 1;
@@ -944,28 +950,32 @@ __device__ __forceinline__ void level_window(const LevelArgs& a, uint64_t window
                     }
                     left = kept;
                 }
+            } else if constexpr (kCarry) {
+                // Carried states first, then the list, in whole waves of 32;
+                // what does not fill one is carried to the next chunk.
+                const uint32_t all = carried + total, run = last ? all : all & ~31u;
+                auto state = [&](uint32_t k) -> uint32_t {  // window offset, operator bits above it
+                    const uint32_t v = wlist[k - carried];
+                    return ch * kChunk + (MODE == kFrontier ? (v & 0x7FFu) | (v >> 11 << 20) : v);
+                };
+                for (uint32_t e = uint32_t(lane); e < run; e += 32) {
+                    const uint32_t v = e < carried ? carry : state(e), o = v & 0xFFFFFu;
+                    em.parent_off = o;
+                    if constexpr (PZ::kSymMult && MODE != kFrontier) {
+                        if (a.sym_mult) mult += PZ::sym_mult(base + o);
+                    }
+                    PZ::template expand<MODE == kFrontier>(base + o, MODE == kFrontier ? v >> 20 : 0u, a.pz, em);
+                }
+                const uint32_t k = run + uint32_t(lane);
+                if (k < all && (run || k >= carried)) carry = state(k);
+                carried = all - run;
             } else
             for (uint32_t e = uint32_t(lane); e < total; e += 32) {
-                if constexpr (MODE == kFrontier) {
-                    const uint32_t v = wlist[e];
-                    em.parent_off = ch * kChunk + (v & 0xFFFFu);
-                    PZ::template expand<true>(cbase + (v & 0xFFFFu), v >> 16, a.pz, em);
-                } else {
-                    em.parent_off = ch * kChunk + wlist[e];
-                    const uint64_t p = cbase + wlist[e];
-                    if constexpr (PZ::kSymMult) {
-                        if (a.sym_mult) mult += PZ::sym_mult(p);
-                    }
-                    if constexpr (kPrefixed) {
-                        uint32_t var;
-                        const uint32_t r = split(p, var);
-                        PZ::template expand_from_prefixed<kFlip3 ? 2 : kPairs ? 1 : 0>(p, pref[var], r, em);
-                    } else if constexpr (kPairs) {
-                        PZ::template expand_from<kFlip3 ? 2 : 1>(p, a.pz, em);
-                    } else {
-                        PZ::template expand<false>(p, 0u, a.pz, em);
-                    }
-                }
+                em.parent_off = ch * kChunk + wlist[e];
+                const uint64_t p = cbase + wlist[e];
+                uint32_t var;
+                const uint32_t r = split(p, var);
+                PZ::template expand_from_prefixed<kFlip3 ? 2 : kPairs ? 1 : 0>(p, pref[var], r, em);
             }
             __syncwarp();
         }
