@@ -434,10 +434,14 @@ struct ExpandPool {
     uint32_t* d_ops_in = nullptr;
     uint64_t* d_out = nullptr;
     uint32_t* d_ops = nullptr;
-    unsigned long long* d_err = nullptr;
+    // Pinned: the kernel sets it for a parent out of range, and the host reads
+    // it after waiting; clearing and copying back a device word was half of a
+    // small call.
+    volatile unsigned long long* h_err = nullptr;
     cudaStream_t stream = nullptr;
     void release() {
-        cudaFree(d_par); cudaFree(d_ops_in); cudaFree(d_out); cudaFree(d_ops); cudaFree(d_err);
+        cudaFree(d_par); cudaFree(d_ops_in); cudaFree(d_out); cudaFree(d_ops);
+        if (h_err) cudaFreeHost(const_cast<unsigned long long*>(h_err));
         if (stream) cudaStreamDestroy(stream);
         *this = ExpandPool();
     }
@@ -458,7 +462,7 @@ int pool_reserve(int branching) {
     PSB_CUDA(cudaMalloc(&g_pool.d_ops_in, kExpandChunk * 4));
     PSB_CUDA(cudaMalloc(&g_pool.d_out, out_cap * 8));
     PSB_CUDA(cudaMalloc(&g_pool.d_ops, out_cap * 4));
-    PSB_CUDA(cudaMalloc(&g_pool.d_err, 8));
+    PSB_CUDA(cudaMallocHost(const_cast<unsigned long long**>(&g_pool.h_err), 8));
     PSB_CUDA(cudaStreamCreateWithFlags(&g_pool.stream, cudaStreamNonBlocking));
     g_pool.cap = kExpandChunk;
     g_pool.out_cap = out_cap;
@@ -514,13 +518,14 @@ int psb_puzzle_create(int kind, int a, int b, psb_puzzle** out) {
     if (!out) return fail(PSB_ERR_ARG, "out is NULL");
     auto p = std::make_unique<psb_puzzle>();
     p->kind = kind; p->a = a; p->b = b;
-    p->pz = PuzzleArgs{0, 0, 0};
+    p->pz = PuzzleArgs{};
     bool ok = false;
     switch (kind) {
     case PSB_SLIDING:  // SlidingTilePuzzleSimple.h:13-19, .cpp:35-39
         if (a < 1 || b < 1 || a * b < 2 || a * b > 16) return fail(PSB_ERR_ARG, "sliding tile %dx%d: need 2 <= w*h <= 16", a, b);
         p->cells = a * b; p->n_states = factorial(a * b); p->ops = 4; p->branching = 4; p->odd = 0;
         p->pz.width = a;
+        p->pz.inv_width = (256 + a - 1) / a;
         ok = psb::sliding_kernels(a * b, &p->k);
         break;
     case PSB_PANCAKE:  // PancakeSimple.h:13-19, .cpp:26,36-40
@@ -545,6 +550,7 @@ int psb_puzzle_create(int kind, int a, int b, psb_puzzle** out) {
             return fail(PSB_ERR_ARG, "sliding tile %dx%d: need 4 <= w*h <= 16", a, b);
         p->cells = a * b; p->n_states = sopt_indexes(a * b); p->ops = 4; p->branching = 4; p->odd = 0;
         p->pz.width = a;
+        p->pz.inv_width = (256 + a - 1) / a;
         ok = psb::sliding_opt_kernels(a * b, &p->k);
         break;
     case PSB_HANOI4:      // FourPegHanoiSimple.h:14-20, .cpp:141-143
@@ -694,18 +700,17 @@ int psb_expand(const psb_puzzle* p, const uint64_t* parents, const uint32_t* opb
     if (int rc = ensure_device(-1)) return rc;
     if (int rc = pool_reserve(p->branching)) return rc;
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : g_pool.stream;
-    PSB_CUDA(cudaMemsetAsync(g_pool.d_err, 0, 8, s));
+    *g_pool.h_err = 0;  // every earlier call of this thread has been waited for
+    unsigned long long* const err = const_cast<unsigned long long*>(g_pool.h_err);
     if (!host) {
         // Device pointers: one launch per chunk, slots written in place.
         for (uint64_t off = 0; off < n; off += kExpandChunk) {
             const uint64_t m = std::min(kExpandChunk, n - off);
             PSB_CUDA(p->k.expand(parents + off, use_ob ? opbits + off : nullptr, m, p->n_states, children + off * br,
-                                 child_ops + off * br, p->pz, g_pool.d_err, use_ob, s));
+                                 child_ops + off * br, p->pz, err, use_ob, s));
         }
-        unsigned long long err = 0;
-        PSB_CUDA(cudaMemcpyAsync(&err, g_pool.d_err, 8, cudaMemcpyDeviceToHost, s));
         PSB_CUDA(cudaStreamSynchronize(s));
-        if (err) return fail(PSB_ERR_ARG, "a parent index is >= IndexesCount()");
+        if (*g_pool.h_err) return fail(PSB_ERR_ARG, "a parent index is >= IndexesCount()");
         *n_out = n * br;
         return PSB_OK;
     }
@@ -719,7 +724,7 @@ int psb_expand(const psb_puzzle* p, const uint64_t* parents, const uint32_t* opb
         PSB_CUDA(cudaMemcpyAsync(g_pool.d_par, parents + off, m * 8, cudaMemcpyHostToDevice, s));
         if (use_ob) PSB_CUDA(cudaMemcpyAsync(g_pool.d_ops_in, opbits + off, m * 4, cudaMemcpyHostToDevice, s));
         PSB_CUDA(p->k.expand(g_pool.d_par, g_pool.d_ops_in, m, p->n_states, g_pool.d_out, g_pool.d_ops, p->pz,
-                             g_pool.d_err, use_ob, s));
+                             err, use_ob, s));
         uint64_t* dst = children + off * br;
         uint32_t* dop = child_ops + off * br;
         if (compact) {

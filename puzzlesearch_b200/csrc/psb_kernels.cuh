@@ -76,6 +76,7 @@ __host__ __device__ constexpr int level_threads(int mode) {
 struct PuzzleArgs {
     int width;  // sliding tile: board width
     int disks;  // Hanoi: number of disks
+    int inv_width;  // sliding tile: ceil(256 / width)
     int sym;    // Hanoi: 0 no symmetry, 1 FourPegHanoiSimple's, 2 FourPegHanoiOptimized's (see Hanoi::expand)
 };
 
@@ -205,11 +206,11 @@ struct SlidingK {
     struct Prefix { uint32_t unused; };
     template <bool kOpBits, class E>
     __device__ __forceinline__ static void expand(uint64_t i, uint32_t ob, const PuzzleArgs& a, E& e) {
-        Sliding<N>::template expand<kOpBits>(i, ob, a.width, e);
+        Sliding<N>::template expand<kOpBits>(i, ob, a.width, a.inv_width, e);
     }
     template <class E>
     __device__ __forceinline__ static void probe_range(uint64_t i, int, int, const PuzzleArgs& a, E& e) {
-        Sliding<N>::template expand<false>(i, 0u, a.width, e);
+        Sliding<N>::template expand<false>(i, 0u, a.width, a.inv_width, e);
     }
 };
 struct HanoiK {
@@ -1124,7 +1125,7 @@ __global__ void __launch_bounds__(kExpandThreads) expand_batch_kernel(const uint
             PZ::template expand<kOpBits>(p, kOpBits ? opbits[i] : 0u, pz, em);
             k = em.k;
         } else {
-            atomicOr(err, 1ull);
+            *err = 1;  // a word of host memory, cleared before the launch
         }
         const uint32_t inv_op = (1u << PZ::kOps) - 1u;
         for (; k < kB; ++k) {

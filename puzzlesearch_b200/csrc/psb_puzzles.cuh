@@ -384,51 +384,56 @@ struct Sliding {
         return D;
     }
 
+    // inv_width = ceil(256 / width), so b / width = b * inv_width >> 8 for b < 16.
     template <bool kOpBits, class Emit>
-    __device__ __forceinline__ static void expand(uint64_t index, uint32_t opbits, int width, Emit& emit) {
+    __device__ __forceinline__ static void expand(uint64_t index, uint32_t opbits, int width, int inv_width,
+                                                  Emit& emit) {
         const uint64_t D = digits(index);
         // first zero digit (the last digit is always 0): the lowest nibble
         // flag is exact, borrows only reach nibbles above a zero one
         constexpr uint64_t kOnes = 0x1111111111111111ull;
         const int b = (__ffsll((long long)((D - kOnes) & ~D & (kOnes << 3))) - 1) >> 2;
-        const int col = b % width;
-        auto digit = [&](int i) -> uint32_t { return uint32_t(D >> (4 * i)) & 15u; };
+        const int col = b - width * ((b * inv_width) >> 8);
+        auto from = [&](int i) -> uint32_t { return uint32_t(D >> (4 * i)); };  // eight digits, i first
         auto weight = [&](int i) -> Delta { return Delta(__ldg(&kFactorials[N - 1 - i])); };
         auto child = [&](Delta delta, uint32_t op) {
             if constexpr (N <= 12 && EmitRel<Emit>::value) emit.rel(index, int32_t(delta), op);
             else if constexpr (N <= 12) emit(index + int64_t(int32_t(delta)), op);
             else emit(index + delta, op);
         };
+        const Delta wb = weight(b);
+        const uint32_t right = from(b + 1 < 16 ? b + 1 : 15);  // the digits right of the blank
         if (b >= width && !(kOpBits && (opbits & 1u))) {
             const int a = b - width;
-            uint32_t R = digit(a) - 1;
-            Delta t = digit(a);  // Horner sum of the digit changes at a .. j
+            uint32_t left = from(a), R = (left & 15u) - 1;
+            Delta t = left & 15u;  // Horner sum of the digit changes at a .. j
             for (int j = a + 1; j < b; ++j) {
-                const uint32_t s = digit(j) <= R ? 1u : 0u;
+                left >>= 4;
+                const uint32_t s = (left & 15u) <= R ? 1u : 0u;
                 R -= s;
                 t = t * Delta(N - j) + s;
             }
-            child(-((t * Delta(N - b) - R) * weight(b)), 3u);
+            child(-((t * Delta(N - b) - R) * wb), 3u);
         }
         if (b < N - width && !(kOpBits && (opbits & 8u))) {
             const int c = b + width;
-            uint32_t r = digit(c);
+            uint32_t r = (right >> (4 * (width - 1))) & 15u;
             Delta w = weight(c), sum = -(Delta(r) * w);
             for (int j = c - 1; j > b; --j) {
                 w *= Delta(N - 1 - j);
-                const uint32_t s = digit(j) <= r ? 1u : 0u;
+                const uint32_t s = ((right >> (4 * (j - b - 1))) & 15u) <= r ? 1u : 0u;
                 r += s;
                 sum += s ? w : Delta(0);
             }
-            child(sum + Delta(r + 1) * w * Delta(N - 1 - b), 0u);
+            child(sum + Delta(r + 1) * wb, 0u);
         }
         if (col > 0 && !(kOpBits && (opbits & 2u))) {
-            const Delta d = digit(b - 1);
-            child(-((d * Delta(N - b) - (d - 1)) * weight(b)), 2u);
+            const Delta d = from(b - 1) & 15u;
+            child(-((d * Delta(N - b) - (d - 1)) * wb), 2u);
         }
         if (col < width - 1 && !(kOpBits && (opbits & 4u))) {
-            const Delta d = digit(b + 1), w = weight(b + 1);
-            child((d + 1) * w * Delta(N - 1 - b) - d * w, 1u);
+            const Delta d = right & 15u;
+            child((d + 1) * wb - d * weight(b + 1), 1u);
         }
     }
 };
