@@ -1277,20 +1277,22 @@ int spill_depth(psb_bfs_session* S, const psb_bfs_opts* o, uint32_t depth, const
     return PSB_OK;
 }
 
-// Runs a whole two-bit search in one launch (psb_small.cuh): S->h_stats holds
+// Runs a whole search in one launch (psb_small.cuh): S->h_stats holds
 // its result afterwards.  *done false: too deep for it, or no cluster of that
 // size here; nothing has happened to the session that a search does not reset.
 int small_search(psb_bfs_session* S, uint64_t initial, uint32_t max_depth, int direction, double ratio, bool can_bu,
-                 bool codes, bool* done) {
+                 bool arrays, bool* done) {
     psb::SmallArgs a{};
     a.n_states = S->p.n_states;
     a.initial = initial;
-    a.codes = codes ? S->arr[0] : nullptr;
-    a.code_words = words_for(2 * S->p.n_states);
+    for (int i = 0; i < S->n_arr; i++) a.arrays[i] = arrays ? S->arr[i] : nullptr;
+    a.units = S->algo == PSB_TWO_BIT ? words_for(2 * S->p.n_states) : 2 * words_for(S->p.n_states);
+    a.mode = S->mode;
     a.out = S->small;
     a.ratio = ratio;
     a.pz = S->p.pz;
-    a.max_levels = max_depth ? max_depth + 1 : 0xFFFFFFFFu;
+    // Two-bit runs the level of the last depth too (it counts the depth).
+    a.max_levels = !max_depth ? 0xFFFFFFFFu : S->algo == PSB_TWO_BIT ? max_depth + 1 : max_depth;
     a.bits = 10;
     while (S->p.n_states > uint64_t(psb::kSmallBlocks) << a.bits) a.bits++;
     a.direction = direction;
@@ -1335,7 +1337,7 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
     // Three-bit needs its visited array; classic (closed) and two-bit (codes) carry the information.
     const bool can_bu = S->bottom_up && direction != PSB_DIR_TOP_DOWN &&
                         (S->algo != PSB_THREE_BIT || S->visited != nullptr);
-    // A small two-bit search with nothing to hand over between its levels
+    // A small search with nothing to hand over between its levels
     // runs in one launch.
     bool whole = false;
     if (S->small && !spill && !restored && !(opts && (opts->level_ms || opts->far_marks || opts->threads))) {
@@ -1438,6 +1440,7 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
             if (opts && opts->level_children && l < cap) opts->level_children[l] = h[psb::kSmallHeader + 2 * l + 1];
             if (count) res.push_back(count);
         }
+        if (S->algo != PSB_TWO_BIT && h[6]) res.push_back(h[6]);  // the depth that the last level found
     }
     while (!whole) {
         if (max_depth && res.size() >= size_t(max_depth) + 1) break;
@@ -1777,7 +1780,7 @@ int psb_bfs_session_create(const psb_puzzle* p, int algo, const psb_bfs_opts* op
     for (auto& f : S->wflags)
         if (int rc = S->alloc(reinterpret_cast<void**>(&f), S->n_windows)) return rc;
     if (int rc = S->alloc(reinterpret_cast<void**>(&S->d_stats), 8 * sizeof(unsigned long long))) return rc;
-    if (algo == PSB_TWO_BIT && p->k.small && S->own_windows &&
+    if (algo != PSB_FRONTIER && p->k.small && S->own_windows &&
         p->n_states <= kSmallChildren / uint64_t(p->branching)) {
         if (int rc = S->alloc(reinterpret_cast<void**>(&S->small), kSmallOut * 8)) return rc;
     }

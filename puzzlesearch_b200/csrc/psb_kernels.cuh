@@ -1245,22 +1245,23 @@ __global__ void __launch_bounds__(kThreads) segment_expand_kernel(SegExpandArgs 
 }
 
 // ---------------------------------------------------------------------------
-// Whole two-bit searches of small puzzles in one launch (psb_small.cuh).
+// Whole searches of small puzzles in one launch (psb_small.cuh).
 // ---------------------------------------------------------------------------
 constexpr int kSmallBlocks = 16, kSmallThreads = 512;
 constexpr uint32_t kSmallDepths = 1024;  // deeper searches run level by level
-constexpr int kSmallHeader = 6;          // words before the depths' (count, children) pairs
+constexpr int kSmallHeader = 7;          // words before the depths' (count, children) pairs
 constexpr int kSmallBottomUp = 2;        // SmallArgs::direction (PSB_DIR_BOTTOM_UP); 0: automatic
 struct SmallArgs {
     uint64_t n_states, initial;
-    uint64_t* codes;          // final two-bit codes (NULL: not wanted)
-    uint64_t code_words;
+    uint64_t* arrays[3];      // final arrays of the search's mode (NULL: not wanted)
+    uint64_t units;           // units of 32 states they have (two-bit: 64-bit words, else 32-bit words)
     unsigned long long* out;  // status (1: bad child, 2: too deep), levels, bottom-up levels, expanded, children,
-                              // local children, then each level's count and children
+                              // local children, the frontier left, then each level's count and children
     double ratio;             // bottom-up below ratio x frontier unvisited states
     PuzzleArgs pz;
     uint32_t max_levels;
     int bits;                 // log2 states per block: kSmallBlocks << bits >= n_states
+    int mode;                 // kTwoBit, kThreeBit or kClassic
     int direction, can_bu;
 };
 using SmallLaunch = cudaError_t (*)(const SmallArgs&, cudaStream_t);

@@ -1,4 +1,5 @@
-// psb_small.cuh -- a whole two-bit search of a small puzzle in one launch.
+// psb_small.cuh -- a whole search (two-bit, three-bit or classic) of a small
+// puzzle in one launch.
 //
 // A level of a small search (3x3 board: at most 24,047 states) is a few
 // microseconds of work, and launching it, clearing its counters, reading them
@@ -69,10 +70,13 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_search_kernel(SmallArg
     const uint32_t rank = cluster.block_rank(), tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t units = 1u << (a.bits - 5);  // 32 states each
     uint32_t *visited = small_mem, *front = visited + units, *marks = front + units;
-    uint16_t* list = reinterpret_cast<uint16_t*>(marks + units) + warp * 1024;
+    // Three-bit's final arrays hold the last two depths.
+    const bool keep = a.mode == kThreeBit && a.arrays[0];
+    uint32_t *prev = marks + units, *before = prev + (keep ? units : 0);
+    uint16_t* list = reinterpret_cast<uint16_t*>(before + (keep ? units : 0)) + warp * 1024;
     const uint64_t n = a.n_states, base = uint64_t(rank) << a.bits;
 
-    for (uint32_t u = tid; u < 3 * units; u += T) small_mem[u] = 0;
+    for (uint32_t u = tid; u < (keep ? 5 : 3) * units; u += T) small_mem[u] = 0;
     if (tid < 4) own[tid] = 0;
     __syncthreads();
     if (tid == 0 && (a.initial >> a.bits) == rank) {
@@ -130,6 +134,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_search_kernel(SmallArg
         for (uint32_t u = tid; u < units; u += T) {
             const uint32_t v = visited[u], f = marks[u] & ~v;
             if (marks[u]) marks[u] = 0;
+            if (keep) {
+                before[u] = prev[u];
+                prev[u] = front[u];
+            }
             front[u] = f;
             if (f) visited[u] = v | f;
             found += __popc(f);
@@ -170,17 +178,28 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_search_kernel(SmallArg
         if (frontier == 0) break;
     }
     if (rank == 0 && tid == 0) {
-        const uint64_t head[kSmallHeader] = {status, level, bu_levels, expanded, children, local};
+        const uint64_t head[kSmallHeader] = {status, level, bu_levels, expanded, children, local, frontier};
         for (int i = 0; i < kSmallHeader; ++i) a.out[i] = head[i];
     }
-    if (a.codes) {
-        // The reference's codes: visited states OLD (1), the last depth's CUR,
-        // 2 at even depths and 3 at odd ones (bit 2i = code / 2, bit 2i + 1 = code % 2).
-        for (uint32_t u = tid; u < units; u += T) {
-            const uint64_t w = (base >> 5) + u;
-            if (w >= a.code_words) break;
+    // The arrays as the level-by-level search leaves them.
+    for (uint32_t u = tid; a.arrays[0] && u < units; u += T) {
+        const uint64_t w = (base >> 5) + u;
+        if (w >= a.units) break;
+        uint32_t* const one[3] = {reinterpret_cast<uint32_t*>(a.arrays[0]), reinterpret_cast<uint32_t*>(a.arrays[1]),
+                                  reinterpret_cast<uint32_t*>(a.arrays[2])};
+        if (a.mode == kTwoBit) {
+            // Codes: visited states OLD (1), the depth that no level expanded
+            // CUR, 2 at even depths and 3 at odd ones (bit 2i = code / 2, bit 2i + 1 = code % 2).
             const uint64_t f = spread_even(front[u]), old = spread_even(visited[u] & ~front[u]);
-            a.codes[w] = f | ((old | ((level & 1) ? f : 0)) << 1);
+            a.arrays[0][w] = f | ((old | ((level & 1) ? f : 0)) << 1);
+        } else if (a.mode == kThreeBit) {  // old, cur: the last two depths; new: empty
+            one[0][w] = frontier ? prev[u] : before[u];
+            one[1][w] = frontier ? front[u] : prev[u];
+            one[2][w] = 0;
+        } else {  // closed, open: the depth that no level expanded, newOpen: empty
+            one[0][w] = visited[u];
+            one[1][w] = front[u];
+            one[2][w] = 0;
         }
     }
     cluster.sync();  // no block leaves while others may still reach into it
@@ -188,7 +207,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_search_kernel(SmallArg
 
 template <class PZ>
 cudaError_t launch_small_search(const SmallArgs& a, cudaStream_t s) {
-    const size_t smem = 3 * (size_t(1) << a.bits) / 8 + kSmallThreads / 32 * 1024 * 2;
+    const size_t bitmaps = a.mode == kThreeBit && a.arrays[0] ? 5 : 3;
+    const size_t smem = bitmaps * (size_t(1) << a.bits) / 8 + kSmallThreads / 32 * 1024 * 2;
     cudaError_t e = cudaFuncSetAttribute(small_search_kernel<PZ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(small_search_kernel<PZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));

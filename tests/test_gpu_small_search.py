@@ -1,4 +1,4 @@
-"""Two-bit searches that run whole in one launch, against the oracle and the
+"""Searches that run whole in one launch, against the oracle and the
 level-by-level path (asked for by window_bits): index spaces from two states
 to the largest that run this way, not multiples of a block's share or of 64,
 all directions, searches stopped part-way, packed indexes and peg symmetry."""
@@ -15,8 +15,9 @@ SPECS = ([["pancake", n, 0] for n in (2, 3, 6, 7, 9)] + [["sliding", w, h] for w
          + [["sliding_opt", 2, 2], ["sliding_opt", 3, 3], ["hanoi4_opt", 8, 1], ["pancake_opt", 8, 0]])
 
 
+@pytest.mark.parametrize("algo", ["two_bit", "three_bit", "classic"])
 @pytest.mark.parametrize("spec", SPECS, ids=lambda s: f"{s[0]}{s[1]}x{s[2]}")
-def test_counts_and_final_arrays(spec):
+def test_counts_and_final_arrays(spec, algo):
     p = make(spec)
     n = p.IndexesCount()
     if spec[0] == "sliding_opt":
@@ -24,14 +25,14 @@ def test_counts_and_final_arrays(spec):
     else:
         starts = {0, n - 1, n * 5 // 7} if not spec[2] or spec[0] == "sliding" else {0}
     for start in starts:
-        counts, final = O.bfs(spec, "two_bit", start, final=True)
+        counts, final = O.bfs(spec, algo, start, final=True)
         for direction in ("auto", "top_down", "bottom_up"):
-            r = psb.bfs(p, "two_bit", start, final=True, direction=direction)
+            r = psb.bfs(p, algo, start, final=True, direction=direction)
             assert r["stats"]["expand_launches"] == 1
             assert r["counts"] == counts and r["final"] == final, direction
         for md in {1, 2, len(counts) // 2, len(counts) - 1, len(counts) + 3} - {0}:
-            r = psb.bfs(p, "two_bit", start, final=True, max_depth=md)
-            want = psb.bfs(p, "two_bit", start, final=True, max_depth=md, window_bits=10)
+            r = psb.bfs(p, algo, start, final=True, max_depth=md)
+            want = psb.bfs(p, algo, start, final=True, max_depth=md, window_bits=10)
             assert want["stats"]["expand_launches"] > 1 or len(counts) == 1 or md < 2
             assert r["counts"] == counts[:md + 1]
             assert r["final"] == want["final"], md
