@@ -11,11 +11,12 @@
 // (direction, end of the search) from counts the blocks exchange.  Global
 // memory sees the final codes and the counts only.  B200, whole calls: 3x3 board
 // 950 -> 232 us (32 levels, 6 us each), 8 pancakes 342 -> 96 us, 8-disk Hanoi
-// 922 -> 306 us.
+// 922 -> 149 us.
 #pragma once
 
 #include <cooperative_groups.h>
 
+#include "psb_hanoi_words.cuh"
 #include "psb_kernels.cuh"
 
 namespace psb {
@@ -42,6 +43,43 @@ struct SmallMarker {
         atomicOr(word, 1u << (o & 31u));
     }
 };
+
+// Hanoi without symmetry, 64 states at a time (psb_hanoi_words.cuh): the
+// children of frontier states F of the block's unit u.  An 8-disk search took
+// 306 us state by state: the warps whose 32 words hold most of a level's states
+// expanded them alone; 149 us.
+__device__ __forceinline__ void small_hanoi_unit(SmallMarker& em, const PuzzleArgs& pz, uint32_t u, uint64_t F) {
+    const uint32_t U = (em.rank << (em.bits - 6)) + u;
+    const uint32_t E = 0x55555555u & ((1u << (2 * (pz.disks - 3))) - 1u);  // a small search has few disks
+    auto mark = [&](uint32_t T, uint64_t m) {
+        const uint32_t owner = T >> (em.bits - 6);
+        uint32_t* word = em.marks + 2 * (T & ((1u << (em.bits - 6)) - 1u));
+        if (owner != em.rank) word = cooperative_groups::this_cluster().map_shared_rank(word, owner);
+        if (uint32_t(m)) atomicOr(word, uint32_t(m));
+        if (uint32_t(m >> 32)) atomicOr(word + 1, uint32_t(m >> 32));
+    };
+    mark(U, unit_moves<kThreeBit, 0>(F) | unit_moves<kThreeBit, 1>(F) | unit_moves<kThreeBit, 2>(F));
+    uint32_t none = 0, elsewhere = 0;  // pairs with both pegs empty; children in other blocks
+#pragma unroll
+    for (uint32_t i = 0; i < 6; ++i) {
+        const uint32_t x = 1 + (i >> 1), v = i & 1;
+        const uint64_t S = F & unit_free_mask<kThreeBit>(int(x), int(v));
+        if (!S) continue;
+        const uint32_t g = x == 1 ? U >> 1 : x == 2 ? U : U ^ (U >> 1);
+        const uint32_t e = (v ? g : ~g) & E, k = e & (0u - e);
+        const uint32_t c = __popcll(S);
+        if (!k) {
+            none += c;
+            continue;
+        }
+        const uint32_t T = U ^ (k * x);
+        if (T >> (em.bits - 6) != em.rank) elsewhere += c;
+        mark(T, S);
+    }
+    const uint32_t children = 6 * __popcll(F) - none;
+    em.children += children;
+    em.local += children - elsewhere;
+}
 
 // Neighbours of an unvisited state: is one of them in the frontier?
 struct SmallProbe {
@@ -94,8 +132,16 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_search_kernel(SmallArg
                                      (a.direction == 0 && frontier >= n / 64 && double(unvisited) < a.ratio * double(frontier)));
         SmallMarker mark{marks, n, rank, a.bits};
         SmallProbe probe{front, n, rank, a.bits};
+        bool by_unit = false;
+        if constexpr (PZ::kSymMult) {
+            by_unit = !bu && hanoi_words_ok(a.pz);
+            for (uint32_t u = tid; by_unit && u < units / 2; u += T) {
+                const uint64_t F = front[2 * u] | (uint64_t(front[2 * u + 1]) << 32);
+                if (F) small_hanoi_unit(mark, a.pz, u, F);
+            }
+        }
         // A warp lists the states of 32 words and expands them 32 at a time.
-        for (uint32_t u0 = warp * 32; u0 < units; u0 += T) {
+        for (uint32_t u0 = warp * 32; !by_unit && u0 < units; u0 += T) {
             const uint32_t u = u0 + lane;
             uint32_t m = bu ? ~visited[u] : front[u];
             if (bu) {  // states below n_states only
