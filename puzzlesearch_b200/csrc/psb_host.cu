@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../include/psb200.h"
+#include "psb_hanoi_words.cuh"
 #include "psb_internal.h"
 #include "psb_kernels.cuh"
 
@@ -873,9 +874,21 @@ struct SpillSeg {
 
 // Searches of up to kSmallChildren children run in one launch, on 16 SMs; larger
 // ones level by level on all of them, a host round trip each.  On B200 (level
-// by level -> one launch): 10-disk Hanoi (6.3 M children) 1.35 -> 1.13 ms, 2x5
-// board (14.5 M) 1.91 -> 1.22 ms, 10 pancakes (32.7 M) 0.63 -> 1.29 ms.
+// by level -> one launch): 2x5 board (14.5 M children) 1.91 -> 1.16 ms, 10
+// pancakes (32.7 M) 0.63 -> 1.29 ms.  Hanoi without symmetry is expanded 64
+// states at a time and goes that way as far as its bitmaps fit the blocks'
+// shared memory (11 disks 2.9 -> 0.8 ms).  A search of bottom-up levels probes
+// for every unvisited state at every level, so it soon wants all SMs: 2x4 board
+// 2.4 -> 1.0 ms, 9 pancakes 0.87 -> 0.90 ms, 2x5 board 5.8 -> 24 ms.
 constexpr uint64_t kSmallChildren = uint64_t(1) << 24;
+constexpr uint64_t kSmallHanoiStates = uint64_t(1) << 22;
+constexpr uint64_t kSmallBottomUpStates = uint64_t(1) << 17;
+
+bool small_states(const psb_puzzle* p) {
+    const bool hanoi = p->kind == PSB_HANOI4 || p->kind == PSB_HANOI4_OPT;
+    if (hanoi && psb::hanoi_words_ok(p->pz)) return p->n_states <= kSmallHanoiStates;
+    return p->n_states <= kSmallChildren / uint64_t(p->branching);
+}
 
 constexpr uint32_t kSpillBatch = 256;  // segments encoded between two waits
 
@@ -1038,10 +1051,10 @@ int layout(const psb_puzzle* p, int algo, uint64_t* words, int* n_arr) {
 constexpr double kBottomUpRatio = 1.0;
 
 // PSB_FAR_AUTO's pick (measured on B200, two-bit, full searches):
-//   13-pancake: ALL 241 ms, NEAR 254 ms, NONE 265 ms;
-//   14-pancake: NEAR 4.18 s, NONE 4.45 s, ALL 4.73 s (its flips of 13 and 14
+//   13-pancake: NEAR 138 ms, NONE 150 ms, ALL 163 ms;
+//   14-pancake: NEAR 2.93 s, NONE 3.03 s, ALL 3.98 s (its flips of 13 and 14
 //   land anywhere in a 10.9 GB bitmap; read-first keeps them read-only);
-//   18-disk Hanoi: NONE 1.58 s, ALL 1.84 s (0.3% of its marks are long-range).
+//   18-disk Hanoi: NONE 0.36 s, ALL 0.46 s (0.3% of its marks are long-range).
 int far_mode(const psb_puzzle* p, int algo, int requested) {
     if (algo != PSB_TWO_BIT) return PSB_FAR_NONE;
     if (requested >= PSB_FAR_NONE && requested <= PSB_FAR_ALL) return requested;
@@ -1055,9 +1068,11 @@ bool supports_bottom_up(const psb_puzzle* p, int algo) {
 }
 
 // Window of 2^16 states for the permutation puzzles and 2^17 for Hanoi
-// (window sweeps on B200: 13-pancake three-bit 353 ms at 2^15..2^16 vs 374 ms
-// at 2^17; 18-disk Hanoi two-bit 1.64 s at 2^17 vs 1.76 s at 2^16), smaller
-// for small puzzles so that every SM gets windows.
+// (swept on B200 with the per-state level kernel: 13-pancake three-bit 353 ms
+// at 2^15..2^16 vs 374 ms at 2^17; 18-disk Hanoi two-bit 1.64 s at 2^17 vs
+// 1.76 s at 2^16), smaller for small puzzles so that every SM gets windows.
+// Top-down levels of 11 and more pancakes have windows of their own
+// (psb_pancake_windows.cuh); theirs is the size of a window flag.
 int auto_window_bits(const psb_puzzle* p, int algo) {
     int lg = 0;
     while (lg < 63 && (uint64_t(1) << (lg + 1)) <= p->n_states) lg++;
@@ -1073,13 +1088,13 @@ size_t smem_bytes(int mode, int wb, int threads = 0) {
 
 // Shape variant of the top-down level kernel for psb_bfs_opts.threads.  With
 // threads = 0, two-bit pancake and Hanoi searches of 2^32 states or more take
-// 128-thread blocks, five per SM (B200 sweeps, whole search, far marks NEAR:
-// 14-pancake 4.06 s at 128 threads vs 4.40 s at 256; 13-pancake 213 vs
-// 219 ms; symmetric 18-disk Hanoi).  Two-bit Hanoi without symmetry (64
-// states at a time, psb_hanoi_words.cuh) takes them at any size: a window's
-// warps finish closer together (17 disks 102 vs 109 ms).  Three-bit
-// (13-pancake 195 vs 193 ms) and the sliding-tile puzzles (3x4 two-bit 45 vs
-// 40 ms) keep 256.
+// 128-thread blocks, five per SM (B200, whole search, far marks NEAR, windows
+// of 2^16: 14-pancake 4.06 s at 128 threads vs 4.40 s at 256).  In windows of
+// 8! states the two are within 2% (14-pancake 2.93 vs 2.86 s, 13-pancake 138
+// vs 135 ms).  Two-bit Hanoi without symmetry (64 states at a time,
+// psb_hanoi_words.cuh) takes them at any size: a window's warps finish closer
+// together (18 disks 358 vs 393 ms).  Three-bit (13-pancake 157 vs 152 ms) and
+// the sliding-tile puzzles (3x4 two-bit 10.5 vs 10.7 ms) keep 256.
 int shape_variant(const psb_puzzle* p, int mode, int threads) {
     if (mode != psb::kTwoBit && mode != psb::kThreeBit) return 0;
     const bool hanoi = p->kind == PSB_HANOI4 || p->kind == PSB_HANOI4_OPT;
@@ -1340,7 +1355,9 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
     // A small search with nothing to hand over between its levels
     // runs in one launch.
     bool whole = false;
-    if (S->small && !spill && !restored && !(opts && (opts->level_ms || opts->far_marks || opts->threads))) {
+    const bool all_bu = can_bu && (direction == PSB_DIR_BOTTOM_UP || bu_ratio > kBottomUpRatio);
+    if (S->small && !spill && !restored && !(opts && (opts->level_ms || opts->far_marks || opts->threads)) &&
+        !(all_bu && N > kSmallBottomUpStates)) {
         if (timed) PSB_CUDA(cudaEventRecord(S->ev[0], s));
         if (int rc = small_search(S, initial, max_depth, direction, bu_ratio, can_bu, opts && opts->final_words, &whole)) return rc;
     }
@@ -1780,8 +1797,7 @@ int psb_bfs_session_create(const psb_puzzle* p, int algo, const psb_bfs_opts* op
     for (auto& f : S->wflags)
         if (int rc = S->alloc(reinterpret_cast<void**>(&f), S->n_windows)) return rc;
     if (int rc = S->alloc(reinterpret_cast<void**>(&S->d_stats), 8 * sizeof(unsigned long long))) return rc;
-    if (algo != PSB_FRONTIER && p->k.small && S->own_windows &&
-        p->n_states <= kSmallChildren / uint64_t(p->branching)) {
+    if (algo != PSB_FRONTIER && p->k.small && S->own_windows && small_states(p)) {
         if (int rc = S->alloc(reinterpret_cast<void**>(&S->small), kSmallOut * 8)) return rc;
     }
     *out = S.release();

@@ -28,7 +28,8 @@ def test_counts_and_final_arrays(spec, algo):
         counts, final = O.bfs(spec, algo, start, final=True)
         for direction in ("auto", "top_down", "bottom_up"):
             r = psb.bfs(p, algo, start, final=True, direction=direction)
-            assert r["stats"]["expand_launches"] == 1
+            if direction != "bottom_up" or spec[2] == 1 or n <= 1 << 17:  # larger bottom-up searches go level by level
+                assert r["stats"]["expand_launches"] == 1
             assert r["counts"] == counts and r["final"] == final, direction
         for md in {1, 2, len(counts) // 2, len(counts) - 1, len(counts) + 3} - {0}:
             r = psb.bfs(p, algo, start, final=True, max_depth=md)
@@ -36,6 +37,18 @@ def test_counts_and_final_arrays(spec, algo):
             assert want["stats"]["expand_launches"] > 1 or len(counts) == 1 or md < 2
             assert r["counts"] == counts[:md + 1]
             assert r["final"] == want["final"], md
+
+
+@pytest.mark.parametrize("algo", ["two_bit", "three_bit", "classic"])
+@pytest.mark.parametrize("disks", [10, 11])
+def test_largest_hanoi(disks, algo):
+    """The largest Hanoi searches that run this way, against the level-by-level path."""
+    p = psb.FourPegHanoiSimple(disks)
+    for start in (0, p.IndexesCount() * 5 // 7):
+        r = psb.bfs(p, algo, start, final=True)
+        want = psb.bfs(p, algo, start, final=True, window_bits=12)
+        assert r["stats"]["expand_launches"] == 1 < want["stats"]["expand_launches"]
+        assert r["counts"] == want["counts"] and r["final"] == want["final"]
 
 
 def test_children_and_sessions():
