@@ -1,24 +1,27 @@
 // psb_kernels.cuh -- sm_100a kernels of the complete-BFS hot path.
 //
 // One level of an in-memory search is ONE fused kernel: each thread block
-// owns an aligned window of 2^window_bits states.  For each window it
-//   1. sweeps the frontier words of the window (coalesced 64-bit loads, one
-//      word per thread), applying the algorithm's sweep-side update
+// owns an aligned window of 2^window_bits states.  For each window its warps
+//   1. sweep the frontier words of the window in chunks of 32 units (coalesced
+//      64-bit loads, one unit per lane), applying the algorithm's sweep-side update
 //      (three-bit: read only; classic: clear open; two-bit: CUR -> OLD with
 //      an atomic XOR; frontier search: clear the 4-bit operator words and
 //      apply the exclusion bitsets);
-//   2. compacts the frontier states of each batch into a shared-memory list
-//      with a block-wide prefix sum, so every thread expands a parent;
-//   3. expands each parent (unrank -> each legal move -> rank) and marks each
+//   2. compact the frontier states of a chunk into the warp's shared-memory
+//      list with a warp prefix sum, so every lane expands a parent;
+//   3. expand each parent (unrank -> each legal move -> rank) and mark each
 //      child: children inside the block's own window go to a shared-memory
 //      bitmap with shared atomics; the rest go straight to global memory
 //      with fire-and-forget atomic ORs (RED);
-//   4. flushes the shared-memory bitmap into global memory, one atomic OR per
+//   4. flush the shared-memory bitmap into global memory, one atomic OR per
 //      non-zero 64-bit word.
 // Puzzle moves are local in index space (a pancake flip of the last k values
 // only changes the last k Lehmer digits; a Hanoi move of disk d only changes
 // bits 2d..2d+1), so most children land in the block's own window and the
-// scattered global traffic shrinks to the long-range moves.
+// scattered global traffic shrinks to the long-range moves.  Two puzzles have
+// level kernels of their own: Hanoi without symmetry (psb_hanoi_words.cuh) and
+// pancakes from 11 on (psb_pancake_windows.cuh); searches of small puzzles run
+// whole in one launch (psb_small.cuh).
 //
 // Array layouts follow the reference exactly (Common/BitArray.h:69-169 and
 // Common/InMemory*.cpp), so final arrays can be compared bit for bit:
@@ -50,9 +53,9 @@ enum Mode : int { kThreeBit = 0, kClassic = 1, kTwoBit = 2, kFrontier = 3 };
 // autotuner's threads-per-block dimension, psb_bfs_opts.threads): 512 and
 // 128 threads per block.  For two-bit they also trade resident warps for
 // registers: 128 per thread at 512 threads (one block per SM), 102 at 128
-// threads (five blocks per SM; B200, whole searches: 13-pancake 213 ms
-// against 226 ms with four blocks of 128 registers, 14-pancake 4.06 s
-// against 4.15 s).  The 13- and 14-pancake kernels issue their far reads
+// threads (five blocks per SM; B200, whole searches in windows of 2^16:
+// 13-pancake 213 ms against 226 ms with four blocks of 128 registers,
+// 14-pancake 4.06 s against 4.15 s).  The 13- and 14-pancake kernels issue their far reads
 // early and keep them in flight across the near children, which needs
 // registers rather than warps (at 64 registers they spill).
 template <int MODE, bool BU = false, int V = 0>
@@ -1161,6 +1164,9 @@ struct SegExpandArgs {
     uint64_t* out;              // cross == 1: children outside the segment
     unsigned long long* out_n;  // cross == 1: entries appended (may exceed out_cap: overflow)
     uint64_t out_cap;
+    unsigned int* hist;         // cross == 1: entries appended per target segment of 2^sb states
+    int sb;
+    uint32_t span;              // words per warp, 1..32
     uint64_t n_states;
     int cross;
     PuzzleArgs pz;
@@ -1187,7 +1193,10 @@ struct SegEmitter {
         unsigned long long base = 0;
         if (lane == leader) base = atomicAdd(a->out_n, (unsigned long long)__popc(mask));
         base = __shfl_sync(mask, base, leader);
-        if (base + rank < a->out_cap) a->out[base + rank] = c;
+        if (base + rank < a->out_cap) {
+            a->out[base + rank] = c;
+            atomicAdd(&a->hist[c >> a->sb], 1u);
+        }
     }
 };
 
@@ -1202,18 +1211,20 @@ __device__ __forceinline__ uint32_t select_bit(uint64_t v, uint32_t k) {
     return pos + ((k >= (w & 1u)) ? 1u : 0u);
 }
 
-// Each warp takes 32 consecutive words of the segment bitmap and expands
+// Each warp takes up to 32 consecutive words of the segment bitmap and expands
 // their set bits 32 at a time, one state per lane: the lanes of a dense word
-// share its states instead of one thread walking all 64.
+// share its states instead of one thread walking all 64.  Fewer words a warp
+// in small segments (segment_span): at 32, the 1024 words of a 2^16-state
+// segment made 32 warps, a handful of SMs working through 100 states a warp.
 template <class PZ>
 __global__ void __launch_bounds__(kThreads) segment_expand_kernel(SegExpandArgs a) {
     SegEmitter em{&a};
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warp = (uint64_t(blockIdx.x) * kThreads + threadIdx.x) >> 5;
     const uint64_t warps = (uint64_t(gridDim.x) * kThreads) >> 5;
-    for (uint64_t w0 = a.word_lo + warp * 32; w0 < a.word_hi; w0 += warps * 32) {
+    for (uint64_t w0 = a.word_lo + warp * a.span; w0 < a.word_hi; w0 += warps * a.span) {
         const uint64_t w = w0 + lane;
-        const uint64_t v = w < a.word_hi ? a.bits[w] : 0;
+        const uint64_t v = lane < a.span && w < a.word_hi ? a.bits[w] : 0;
         const uint32_t c = __popcll(v);
         uint32_t incl = c;  // inclusive prefix of the lanes' set bits
 #pragma unroll

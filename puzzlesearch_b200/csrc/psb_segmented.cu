@@ -60,14 +60,9 @@ __global__ void __launch_bounds__(kThreads) seg_set_offsets(uint64_t* __restrict
     }
 }
 
-// Partition of cross-segment children by target segment: a histogram, then
-// a scatter of each child's offset into its segment's run (order within a
+// Partition of cross-segment children by target segment (counted as they were
+// appended): each child's offset goes into its segment's run (order within a
 // run does not matter: the offsets are ORed into a bitmap).
-__global__ void __launch_bounds__(kThreads) seg_histogram(const uint64_t* __restrict__ kids, uint64_t n, int sb,
-                                                         unsigned int* __restrict__ hist) {
-    for (uint64_t i = blockIdx.x * uint64_t(kThreads) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * kThreads)
-        atomicAdd(&hist[kids[i] >> sb], 1u);
-}
 __global__ void __launch_bounds__(kThreads) seg_scatter(const uint64_t* __restrict__ kids, uint64_t n, int sb,
                                                        unsigned int* __restrict__ cursor,
                                                        uint32_t* __restrict__ out) {
@@ -95,6 +90,8 @@ namespace {
 // buffers, Common/Multiplexor.cpp:5-33), fewer when there are many segments.
 constexpr uint64_t kStageMax = 16384;
 constexpr uint64_t kStageBudget = uint64_t(1) << 26;  // bytes of staging over all segments
+constexpr uint64_t kExpandWarps = 148 * 16;           // warps an expansion is spread over before a warp takes more words
+constexpr uint64_t kPinned = uint64_t(1) << 19;       // longer layers and runs of children go through pageable memory
 
 template <class T>
 struct DevBuf {
@@ -129,6 +126,12 @@ struct Run {
     std::vector<uint8_t> host_stream;    // one layer between the store and the device
     std::vector<psb_codec_block> blocks;
     std::vector<uint32_t> host_offs;     // cross-segment children between the device and the staging
+    // Pinned: counts the device hands over ([0] states found, [1] children),
+    // the children per segment and where their runs start, and up to kPinned
+    // bytes each of a layer and of children on their way to the stores.
+    unsigned long long* pin = nullptr;
+    unsigned int *pin_hist = nullptr, *pin_start = nullptr;
+    uint8_t *pin_stream = nullptr, *pin_offs = nullptr;
     // Multiplexor staging: per target segment, the offsets not yet written.
     uint64_t stage_cap = 0;
     std::vector<uint32_t> stage;
@@ -141,6 +144,20 @@ struct Run {
         if (enc) psb::encoder_destroy(enc);
         if (dec) psb::decoder_destroy(dec);  // frees its scratch in stream order
         if (s) cudaStreamDestroy(s);
+        if (pin) cudaFreeHost(pin);
+    }
+
+    int pin_host() {
+        const uint64_t runs = (n_segments + 3) / 4 * 16;
+        void* v = nullptr;
+        SG_CUDA(cudaMallocHost(&v, 16 + 2 * runs + 2 * kPinned));
+        pin = static_cast<unsigned long long*>(v);
+        uint8_t* at = static_cast<uint8_t*>(v) + 16;
+        pin_hist = reinterpret_cast<unsigned int*>(at);
+        pin_start = reinterpret_cast<unsigned int*>(at + runs);
+        pin_stream = at + 2 * runs;
+        pin_offs = pin_stream + kPinned;
+        return PSB_OK;
     }
 
     uint64_t states_in(uint64_t g) const { return std::min(seg_states, P->n_states - g * seg_states); }
@@ -168,31 +185,6 @@ struct Run {
         st.h2d_bytes += bytes;
         return psb::frontier_decode_async(stream_buf[slot].p, blocks.data(), nb, bits, states_in(g), scalars.p + 3,
                                           dec, s);
-    }
-
-    // Encodes a segment bitmap holding `count` states as segment g's layer in `store`.
-    int encode(const uint64_t* bits, uint64_t g, uint64_t count, psb::StoreImpl& store) {
-        if (count == 0) return PSB_OK;
-        unsigned long long* sums = nullptr;
-        if (int rc = psb::encoder_begin(enc, std::min(seg_states, P->n_states), 1, s, &sums)) return rc;
-        psb::EncTotals t{};
-        for (;;) {  // again with longer buffers if the segment outgrows them
-            if (int rc = psb::encoder_segment(enc, bits, states_in(g), false, 0, 0, stream_buf[0].p,
-                                              stream_buf[0].cap, s))
-                return rc;
-            bool complete = false;
-            if (int rc = psb::encoder_totals(enc, 1, &t, &complete, s)) return rc;
-            if (complete && t.bytes <= stream_buf[0].cap) break;
-            if (complete)
-                if (int rc = stream_buf[0].grow(t.bytes)) return rc;
-        }
-        const uint64_t bytes = t.bytes;
-        if (t.count != count) return psb_set_error(PSB_ERR_DEVICE, "segmented search: layer count mismatch");
-        if (host_stream.size() < bytes) host_stream.resize(bytes);
-        SG_CUDA(cudaMemcpyAsync(host_stream.data(), stream_buf[0].p, bytes, cudaMemcpyDeviceToHost, s));
-        SG_CUDA(cudaStreamSynchronize(s));
-        st.d2h_bytes += bytes;
-        return psb::store_write(store, int(g), host_stream.data(), bytes);
     }
 
     // ORs the offsets segment g received (its chunks in `store`) into `bits`,
@@ -245,11 +237,9 @@ struct Run {
         return PSB_OK;
     }
 
-    // Expands the states of `bits` (segment g) chunk by chunk: with no store
-    // it marks the children inside g in `next`; with one it stages the
-    // offsets of the children outside g for their target segments.
-    int expand(const uint64_t* bits, uint64_t g, psb::StoreImpl* cross_store) {
-        const int cross = cross_store != nullptr;
+    // Expands words w.. of `bits` (segment g), a chunk: its children inside g are
+    // marked in `next`, or (cross) those outside g appended to `kids` and counted per segment.
+    int expand(const uint64_t* bits, uint64_t g, uint64_t w, bool cross) {
         psb::SegExpandArgs a{};
         a.bits = bits;
         a.seg_base = g * seg_states;
@@ -258,46 +248,97 @@ struct Run {
         a.out = kids.p;
         a.out_n = scalars.p + 1;
         a.out_cap = kids.cap;
+        a.hist = hist.p;
+        a.sb = sb;
         a.n_states = P->n_states;
         a.cross = cross;
         a.pz = P->pz;
         a.err = scalars.p + 2;
-        std::vector<unsigned int> h(cross ? n_segments : 0), start(cross ? n_segments : 0);
-        for (uint64_t w = 0; w < seg_words; w += chunk_words) {
-            a.word_lo = w;
-            a.word_hi = std::min(seg_words, w + chunk_words);
+        a.word_lo = w;
+        a.word_hi = std::min(seg_words, w + chunk_words);
+        const uint64_t words = a.word_hi - w;
+        a.span = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(32, words / kExpandWarps)));
+        const uint64_t warps = (words + a.span - 1) / a.span;
+        const unsigned grid = unsigned(std::min<uint64_t>((warps * 32 + psb::kThreads - 1) / psb::kThreads, 148 * 8));
+        if (cross) {
             SG_CUDA(cudaMemsetAsync(scalars.p + 1, 0, 8, s));
-            // one warp per 32 words
-            const uint64_t warps = (a.word_hi - w + 31) / 32;
-            const unsigned grid = unsigned(std::min<uint64_t>((warps * 32 + psb::kThreads - 1) / psb::kThreads, 148 * 8));
-            SG_CUDA(P->k.segment_expand(a, grid, s));
-            if (!cross) continue;
-            unsigned long long n = 0;
-            SG_CUDA(cudaMemcpyAsync(&n, scalars.p + 1, 8, cudaMemcpyDeviceToHost, s));
-            SG_CUDA(cudaStreamSynchronize(s));
-            if (n > kids.cap) return psb_set_error(PSB_ERR_DEVICE, "segmented search: child buffer overflow");
-            if (n == 0) continue;
-            st.cross_children += n;
             SG_CUDA(cudaMemsetAsync(hist.p, 0, n_segments * 4, s));
-            const unsigned pg = unsigned(std::min<uint64_t>((n + psb::kThreads - 1) / psb::kThreads, 148 * 16));
-            psb::seg_histogram<<<pg, psb::kThreads, 0, s>>>(kids.p, n, sb, hist.p);
-            SG_CUDA(cudaMemcpyAsync(h.data(), hist.p, n_segments * 4, cudaMemcpyDeviceToHost, s));
-            SG_CUDA(cudaStreamSynchronize(s));
-            unsigned int acc = 0;
-            for (uint64_t t = 0; t < n_segments; t++) { start[t] = acc; acc += h[t]; }
-            SG_CUDA(cudaMemcpyAsync(hist.p, start.data(), n_segments * 4, cudaMemcpyHostToDevice, s));
-            if (int rc = offs.grow(n)) return rc;
-            psb::seg_scatter<<<pg, psb::kThreads, 0, s>>>(kids.p, n, sb, hist.p, offs.p);
-            SG_CUDA(cudaGetLastError());
-            if (host_offs.size() < n) host_offs.resize(n);
-            SG_CUDA(cudaMemcpyAsync(host_offs.data(), offs.p, n * 4, cudaMemcpyDeviceToHost, s));
-            SG_CUDA(cudaStreamSynchronize(s));
-            st.d2h_bytes += n * 4;
-            for (uint64_t t = 0; t < n_segments; t++)
-                if (h[t])
-                    if (int rc = stage_add(*cross_store, t, host_offs.data() + start[t], h[t])) return rc;
         }
-        SG_CUDA(cudaStreamSynchronize(s));
+        SG_CUDA(P->k.segment_expand(a, grid, s));
+        if (cross) {
+            SG_CUDA(cudaMemcpyAsync(pin + 1, scalars.p + 1, 8, cudaMemcpyDeviceToHost, s));
+            SG_CUDA(cudaMemcpyAsync(pin_hist, hist.p, n_segments * 4, cudaMemcpyDeviceToHost, s));
+        }
+        return PSB_OK;
+    }
+    int expand_inside(const uint64_t* bits, uint64_t g) {
+        for (uint64_t w = 0; w < seg_words; w += chunk_words)
+            if (int rc = expand(bits, g, w, false)) return rc;
+        return PSB_OK;
+    }
+
+    // The `count` states of `bits` become segment g's layer in `store`, and the
+    // offsets of their children outside g are staged for their target segments
+    // in `cross_store`.  The host waits twice: for the sizes of the layer and of
+    // the first chunk's children, and for both (it waited seven times when each
+    // size was asked for when it was needed: 10-disk Hanoi in 16 segments, 50
+    // depths, 119 -> 88 to 97 ms).
+    int found(const uint64_t* bits, uint64_t g, uint64_t count, psb::StoreImpl& store, psb::StoreImpl& cross_store) {
+        if (count == 0) return PSB_OK;
+        unsigned long long* sums = nullptr;
+        if (int rc = psb::encoder_begin(enc, std::min(seg_states, P->n_states), 1, s, &sums)) return rc;
+        psb::EncTotals t{};
+        for (bool first = true;; first = false) {  // again with longer buffers if the segment outgrows them
+            if (int rc = psb::encoder_segment(enc, bits, states_in(g), false, 0, 0, stream_buf[0].p,
+                                              stream_buf[0].cap, s))
+                return rc;
+            if (first)
+                if (int rc = expand(bits, g, 0, true)) return rc;
+            bool complete = false;
+            if (int rc = psb::encoder_totals(enc, 1, &t, &complete, s)) return rc;
+            if (complete && t.bytes <= stream_buf[0].cap) break;
+            if (complete)
+                if (int rc = stream_buf[0].grow(t.bytes)) return rc;
+        }
+        if (t.count != count) return psb_set_error(PSB_ERR_DEVICE, "segmented search: layer count mismatch");
+        const bool pinned = t.bytes <= kPinned;
+        if (!pinned && host_stream.size() < t.bytes) host_stream.resize(t.bytes);
+        uint8_t* const layer = pinned ? pin_stream : host_stream.data();
+        SG_CUDA(cudaMemcpyAsync(layer, stream_buf[0].p, t.bytes, cudaMemcpyDeviceToHost, s));
+        st.d2h_bytes += t.bytes;
+        for (uint64_t w = 0; w < seg_words; w += chunk_words) {
+            if (w) {
+                if (int rc = expand(bits, g, w, true)) return rc;
+                SG_CUDA(cudaStreamSynchronize(s));
+            }
+            const uint64_t n = pin[1];
+            if (n > kids.cap) return psb_set_error(PSB_ERR_DEVICE, "segmented search: child buffer overflow");
+            const uint32_t* kids_host = reinterpret_cast<const uint32_t*>(pin_offs);
+            if (n) {
+                st.cross_children += n;
+                unsigned int acc = 0;
+                for (uint64_t i = 0; i < n_segments; i++) { pin_start[i] = acc; acc += pin_hist[i]; }
+                SG_CUDA(cudaMemcpyAsync(hist.p, pin_start, n_segments * 4, cudaMemcpyHostToDevice, s));
+                if (int rc = offs.grow(n)) return rc;
+                const unsigned pg = unsigned(std::min<uint64_t>((n + psb::kThreads - 1) / psb::kThreads, 148 * 16));
+                psb::seg_scatter<<<pg, psb::kThreads, 0, s>>>(kids.p, n, sb, hist.p, offs.p);
+                SG_CUDA(cudaGetLastError());
+                void* to = pin_offs;
+                if (n * 4 > kPinned) {
+                    if (host_offs.size() < n) host_offs.resize(n);
+                    to = host_offs.data();
+                    kids_host = host_offs.data();
+                }
+                SG_CUDA(cudaMemcpyAsync(to, offs.p, n * 4, cudaMemcpyDeviceToHost, s));
+                st.d2h_bytes += n * 4;
+            }
+            if (n || w == 0) SG_CUDA(cudaStreamSynchronize(s));
+            if (w == 0)
+                if (int rc = psb::store_write(store, int(g), layer, t.bytes)) return rc;
+            for (uint64_t i = 0; n && i < n_segments; i++)
+                if (pin_hist[i])
+                    if (int rc = stage_add(cross_store, i, kids_host + pin_start[i], pin_hist[i])) return rc;
+        }
         return PSB_OK;
     }
 };
@@ -368,6 +409,7 @@ extern "C" int psb_bfs_segmented(const psb_puzzle* p, uint64_t initial, const ps
     R.kids.cap = R.chunk_words * 64 * uint64_t(p->branching);
     if (int rc = R.offs.grow(uint64_t(1) << 22)) return rc;
     if (int rc = R.hist.grow(R.n_segments)) return rc;
+    if (int rc = R.pin_host()) return rc;
     if (int rc = R.scalars.grow(4)) return rc;
     if (int rc = R.stream_buf[0].grow(uint64_t(1) << 20)) return rc;
     if (!(R.enc = psb::encoder_create())) return psb_set_error(PSB_ERR_NOMEM, "segmented search: encoder");
@@ -383,9 +425,8 @@ extern "C" int psb_bfs_segmented(const psb_puzzle* p, uint64_t initial, const ps
         const uint64_t off = initial - g0 * R.seg_states;
         const uint64_t word = uint64_t(1) << (off & 63);
         SG_CUDA(cudaMemcpyAsync(R.next.p + off / 64, &word, 8, cudaMemcpyHostToDevice, R.s));
-        if (int rc = R.encode(R.next.p, g0, 1, *cur_s)) return rc;
+        if (int rc = R.found(R.next.p, g0, 1, *cur_s, *recv_s)) return rc;
         cnt_cur[g0] = 1;
-        if (int rc = R.expand(R.next.p, g0, recv_s)) return rc;
         if (int rc = R.stage_flush(*recv_s)) return rc;
     }
     std::vector<uint64_t> res{1};
@@ -404,22 +445,20 @@ extern "C" int psb_bfs_segmented(const psb_puzzle* p, uint64_t initial, const ps
             if (int rc = R.receive(*recv_s, g, R.next.p)) return rc;
             if (int rc = R.decode(*cur_s, R.cur.p, g, 0)) return rc;
             if (cnt_cur[g])
-                if (int rc = R.expand(R.cur.p, g, nullptr)) return rc;
+                if (int rc = R.expand_inside(R.cur.p, g)) return rc;
             if (int rc = R.decode(*old_s, R.old.p, g, 1)) return rc;
             SG_CUDA(cudaMemsetAsync(R.scalars.p, 0, 8, R.s));
             psb::seg_finish<<<148 * 8, psb::kThreads, 0, R.s>>>(R.next.p, R.old.p, R.cur.p, R.seg_words, odd ? 1 : 0,
                                                                R.scalars.p);
             SG_CUDA(cudaGetLastError());
-            unsigned long long c = 0;
-            SG_CUDA(cudaMemcpyAsync(&c, R.scalars.p, 8, cudaMemcpyDeviceToHost, R.s));
+            SG_CUDA(cudaMemcpyAsync(R.pin, R.scalars.p, 8, cudaMemcpyDeviceToHost, R.s));
             SG_CUDA(cudaStreamSynchronize(R.s));
+            const uint64_t c = R.pin[0];
             // g's depth d-1 layer is no longer needed (DeleteSegment of the old layer)
             if (int rc = psb::store_erase(*old_s, int(g))) return rc;
             total += c;
             cnt_new[g] = c;
-            if (int rc = R.encode(R.next.p, g, c, *new_s)) return rc;
-            if (c)
-                if (int rc = R.expand(R.next.p, g, next_s)) return rc;
+            if (int rc = R.found(R.next.p, g, c, *new_s, *next_s)) return rc;
             const uint64_t held = store_bytes();
             (R.files ? R.st.peak_disk_bytes : R.st.peak_host_bytes) =
                 std::max(R.files ? R.st.peak_disk_bytes : R.st.peak_host_bytes, held);
