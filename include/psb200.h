@@ -257,7 +257,8 @@ int psb_bfs_session_destroy(psb_bfs_session* s);
  * that keeps freed memory reserved for the next search instead of returning
  * it to the driver after every call.  This returns the reserved memory of
  * `device` (-1 = current) to the driver, and frees the frontier spill's
- * cached buffers; it waits for the device first. */
+ * cached buffers and the streams, events and pinned words kept for the next
+ * searches (at most 8 sets a device); it waits for the device first. */
 int psb_release_cached_memory(int device);
 
 /* --- Device bit arrays (Common/BitArray.h:69-169) -------------------------
