@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <memory>
 #include <new>
 #include <string>
@@ -390,7 +391,7 @@ struct DecodeScratch {
     uint8_t* buf = nullptr;
     size_t cap = 0;
     cudaStream_t stream = nullptr;
-    std::vector<uint32_t> h_first;
+    std::vector<uint8_t> h_table;  // the blocks, then each one's first tile
 
     int reserve(size_t need, cudaStream_t s) {
         if (need <= cap) return PSB_OK;
@@ -413,20 +414,6 @@ int frontier_decode_async(const uint8_t* d_in, const psb_codec_block* h_blocks, 
                           uint64_t n_bits, unsigned long long* d_err, DecodeScratch* x, cudaStream_t s) {
     if (n_blocks == 0) return PSB_OK;
     // Tiles per block (none for a StreamVInt block without tuples).
-    x->h_first.resize(size_t(n_blocks) + 1);
-    uint64_t n_tiles = 0;
-    bool any_svi = false;
-    for (uint32_t b = 0; b < n_blocks; ++b) {
-        x->h_first[b] = uint32_t(n_tiles);
-        const uint64_t head = h_blocks[b].is_bitmap ? 8 : 4;
-        const uint64_t left = h_blocks[b].bytes > head ? h_blocks[b].bytes - head : 0;
-        uint64_t tiles = (left + kTile - 1) / kTile;
-        if (h_blocks[b].is_bitmap) tiles = std::max<uint64_t>(tiles, 1);  // the first offset is in the header
-        else any_svi = true;
-        n_tiles += tiles;
-        if (n_tiles > 0x7FFFFFFFull) return psb_set_error(PSB_ERR_ARG, "stream too large");
-    }
-    x->h_first[n_blocks] = uint32_t(n_tiles);
     size_t need = 0;
     auto part = [&](size_t bytes) {
         const size_t at = need;
@@ -435,6 +422,23 @@ int frontier_decode_async(const uint8_t* d_in, const psb_codec_block* h_blocks, 
     };
     const size_t at_blocks = part(size_t(n_blocks) * sizeof(psb_codec_block));
     const size_t at_first = part((size_t(n_blocks) + 1) * 4);
+    const size_t table = need;
+    x->h_table.resize(table);
+    std::memcpy(x->h_table.data() + at_blocks, h_blocks, size_t(n_blocks) * sizeof(psb_codec_block));
+    uint32_t* const h_first = reinterpret_cast<uint32_t*>(x->h_table.data() + at_first);
+    uint64_t n_tiles = 0;
+    bool any_svi = false;
+    for (uint32_t b = 0; b < n_blocks; ++b) {
+        h_first[b] = uint32_t(n_tiles);
+        const uint64_t head = h_blocks[b].is_bitmap ? 8 : 4;
+        const uint64_t left = h_blocks[b].bytes > head ? h_blocks[b].bytes - head : 0;
+        uint64_t tiles = (left + kTile - 1) / kTile;
+        if (h_blocks[b].is_bitmap) tiles = std::max<uint64_t>(tiles, 1);  // the first offset is in the header
+        else any_svi = true;
+        n_tiles += tiles;
+        if (n_tiles > 0x7FFFFFFFull) return psb_set_error(PSB_ERR_ARG, "stream too large");
+    }
+    h_first[n_blocks] = uint32_t(n_tiles);
     const size_t at_maps = part(n_tiles * kMapStride), at_entries = part(n_tiles);
     const size_t at_pieces = part(n_tiles * kDT * sizeof(PieceInfo)), at_tiles = part(n_tiles * sizeof(TileInfo));
     if (int rc = x->reserve(need, s)) return rc;
@@ -444,8 +448,8 @@ int frontier_decode_async(const uint8_t* d_in, const psb_codec_block* h_blocks, 
     auto* entries = x->buf + at_entries;
     auto* pieces = reinterpret_cast<PieceInfo*>(x->buf + at_pieces);
     auto* tiles = reinterpret_cast<TileInfo*>(x->buf + at_tiles);
-    DC_CUDA(cudaMemcpyAsync(blocks, h_blocks, size_t(n_blocks) * sizeof(psb_codec_block), cudaMemcpyHostToDevice, s));
-    DC_CUDA(cudaMemcpyAsync(first, x->h_first.data(), (size_t(n_blocks) + 1) * 4, cudaMemcpyHostToDevice, s));
+    // Pageable source: the copy has left host memory when the call returns.
+    DC_CUDA(cudaMemcpyAsync(x->buf, x->h_table.data(), table, cudaMemcpyHostToDevice, s));
     const unsigned grid = unsigned(n_tiles);
     if (any_svi) {
         if (grid) k_tile_maps<<<grid, kDT, 0, s>>>(d_in, blocks, n_blocks, first, maps);

@@ -116,18 +116,18 @@ struct Run {
     int sb = 0;
     uint64_t seg_states = 0, seg_words = 0, n_segments = 0;
     uint64_t chunk_words = 0;
-    DevBuf<uint64_t> next, cur, old, kids;
+    DevBuf<uint64_t> maps, kids;
+    uint64_t *next = nullptr, *cur = nullptr, *old = nullptr;  // the segment's bitmaps, in `maps`
     DevBuf<uint32_t> offs;
     DevBuf<uint8_t> stream_buf[2];  // the two layers decoded for one segment
-    DevBuf<unsigned int> hist;
-    DevBuf<unsigned long long> scalars;  // [0] count, [1] children appended, [2] error flag, [3] decode error
+    DevBuf<unsigned long long> tally;    // [0] states found, [1] children appended, then (32 bits each) those per segment
+    DevBuf<unsigned long long> scalars;  // [0] error flag, [1] decode error
     psb::SegmentEncoder* enc = nullptr;  // device scratch kept from segment to segment
     psb::DecodeScratch* dec = nullptr;
     std::vector<uint8_t> host_stream;    // one layer between the store and the device
     std::vector<psb_codec_block> blocks;
     std::vector<uint32_t> host_offs;     // cross-segment children between the device and the staging
-    // Pinned: counts the device hands over ([0] states found, [1] children),
-    // the children per segment and where their runs start, and up to kPinned
+    // Pinned: the tally, where the children's runs start, and up to kPinned
     // bytes each of a layer and of children on their way to the stores.
     unsigned long long* pin = nullptr;
     unsigned int *pin_hist = nullptr, *pin_start = nullptr;
@@ -148,26 +148,27 @@ struct Run {
     }
 
     int pin_host() {
-        const uint64_t runs = (n_segments + 3) / 4 * 16;
+        const uint64_t tally = (tally_bytes() + 15) / 16 * 16, runs = (n_segments + 3) / 4 * 16;
         void* v = nullptr;
-        SG_CUDA(cudaMallocHost(&v, 16 + 2 * runs + 2 * kPinned));
+        SG_CUDA(cudaMallocHost(&v, tally + runs + 2 * kPinned));
         pin = static_cast<unsigned long long*>(v);
-        uint8_t* at = static_cast<uint8_t*>(v) + 16;
-        pin_hist = reinterpret_cast<unsigned int*>(at);
-        pin_start = reinterpret_cast<unsigned int*>(at + runs);
-        pin_stream = at + 2 * runs;
+        pin_hist = reinterpret_cast<unsigned int*>(pin + 2);
+        pin_start = reinterpret_cast<unsigned int*>(static_cast<uint8_t*>(v) + tally);
+        pin_stream = static_cast<uint8_t*>(v) + tally + runs;
         pin_offs = pin_stream + kPinned;
         return PSB_OK;
     }
 
     uint64_t states_in(uint64_t g) const { return std::min(seg_states, P->n_states - g * seg_states); }
 
+    unsigned int* hist() const { return reinterpret_cast<unsigned int*>(tally.p + 2); }
+    uint64_t tally_bytes() const { return 16 + n_segments * 4; }
+
     // Decodes segment g's layer from `store` into a cleared segment bitmap
     // (slot 0 or 1: the two layers of one segment are in flight together).
-    // Nothing waits on the device: a bad offset sets scalars[3], read at the
+    // Nothing waits on the device: a bad offset sets scalars[1], read at the
     // end of the depth.
     int decode(psb::StoreImpl& store, uint64_t* bits, uint64_t g, int slot) {
-        SG_CUDA(cudaMemsetAsync(bits, 0, seg_words * 8, s));
         const uint64_t bytes = psb::store_length(store, int(g));
         if (bytes == 0) return PSB_OK;
         if (host_stream.size() < bytes) host_stream.resize(bytes);
@@ -183,7 +184,7 @@ struct Run {
         // Pageable source: the copy has left host memory when the call returns.
         SG_CUDA(cudaMemcpyAsync(stream_buf[slot].p, host_stream.data(), bytes, cudaMemcpyHostToDevice, s));
         st.h2d_bytes += bytes;
-        return psb::frontier_decode_async(stream_buf[slot].p, blocks.data(), nb, bits, states_in(g), scalars.p + 3,
+        return psb::frontier_decode_async(stream_buf[slot].p, blocks.data(), nb, bits, states_in(g), scalars.p + 1,
                                           dec, s);
     }
 
@@ -244,31 +245,26 @@ struct Run {
         a.bits = bits;
         a.seg_base = g * seg_states;
         a.seg_states = states_in(g);
-        a.next = next.p;
+        a.next = next;
         a.out = kids.p;
-        a.out_n = scalars.p + 1;
+        a.out_n = tally.p + 1;
         a.out_cap = kids.cap;
-        a.hist = hist.p;
+        a.hist = hist();
         a.sb = sb;
         a.n_states = P->n_states;
         a.cross = cross;
         a.pz = P->pz;
-        a.err = scalars.p + 2;
+        a.err = scalars.p;
         a.word_lo = w;
         a.word_hi = std::min(seg_words, w + chunk_words);
         const uint64_t words = a.word_hi - w;
         a.span = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(32, words / kExpandWarps)));
         const uint64_t warps = (words + a.span - 1) / a.span;
         const unsigned grid = unsigned(std::min<uint64_t>((warps * 32 + psb::kThreads - 1) / psb::kThreads, 148 * 8));
-        if (cross) {
-            SG_CUDA(cudaMemsetAsync(scalars.p + 1, 0, 8, s));
-            SG_CUDA(cudaMemsetAsync(hist.p, 0, n_segments * 4, s));
-        }
+        // The tally is clear before a segment's first chunk.
+        if (cross && w) SG_CUDA(cudaMemsetAsync(tally.p, 0, tally_bytes(), s));
         SG_CUDA(P->k.segment_expand(a, grid, s));
-        if (cross) {
-            SG_CUDA(cudaMemcpyAsync(pin + 1, scalars.p + 1, 8, cudaMemcpyDeviceToHost, s));
-            SG_CUDA(cudaMemcpyAsync(pin_hist, hist.p, n_segments * 4, cudaMemcpyDeviceToHost, s));
-        }
+        if (cross) SG_CUDA(cudaMemcpyAsync(pin, tally.p, tally_bytes(), cudaMemcpyDeviceToHost, s));
         return PSB_OK;
     }
     int expand_inside(const uint64_t* bits, uint64_t g) {
@@ -318,10 +314,10 @@ struct Run {
                 st.cross_children += n;
                 unsigned int acc = 0;
                 for (uint64_t i = 0; i < n_segments; i++) { pin_start[i] = acc; acc += pin_hist[i]; }
-                SG_CUDA(cudaMemcpyAsync(hist.p, pin_start, n_segments * 4, cudaMemcpyHostToDevice, s));
+                SG_CUDA(cudaMemcpyAsync(hist(), pin_start, n_segments * 4, cudaMemcpyHostToDevice, s));
                 if (int rc = offs.grow(n)) return rc;
                 const unsigned pg = unsigned(std::min<uint64_t>((n + psb::kThreads - 1) / psb::kThreads, 148 * 16));
-                psb::seg_scatter<<<pg, psb::kThreads, 0, s>>>(kids.p, n, sb, hist.p, offs.p);
+                psb::seg_scatter<<<pg, psb::kThreads, 0, s>>>(kids.p, n, sb, hist(), offs.p);
                 SG_CUDA(cudaGetLastError());
                 void* to = pin_offs;
                 if (n * 4 > kPinned) {
@@ -403,29 +399,32 @@ extern "C" int psb_bfs_segmented(const psb_puzzle* p, uint64_t initial, const ps
     };
 
     SG_CUDA(cudaStreamCreateWithFlags(&R.s, cudaStreamNonBlocking));
-    for (auto* b : {&R.next, &R.cur, &R.old})
-        if (int rc = b->grow(R.seg_words)) return rc;
+    if (int rc = R.maps.grow(3 * R.seg_words)) return rc;
+    R.next = R.maps.p;
+    R.cur = R.next + R.seg_words;
+    R.old = R.cur + R.seg_words;
     if (int rc = R.kids.grow(R.chunk_words * 64 * uint64_t(p->branching))) return rc;
     R.kids.cap = R.chunk_words * 64 * uint64_t(p->branching);
     if (int rc = R.offs.grow(uint64_t(1) << 22)) return rc;
-    if (int rc = R.hist.grow(R.n_segments)) return rc;
+    if (int rc = R.tally.grow(2 + (R.n_segments + 1) / 2)) return rc;
     if (int rc = R.pin_host()) return rc;
-    if (int rc = R.scalars.grow(4)) return rc;
+    if (int rc = R.scalars.grow(2)) return rc;
     if (int rc = R.stream_buf[0].grow(uint64_t(1) << 20)) return rc;
     if (!(R.enc = psb::encoder_create())) return psb_set_error(PSB_ERR_NOMEM, "segmented search: encoder");
     if (!(R.dec = psb::decoder_create())) return psb_set_error(PSB_ERR_NOMEM, "segmented search: decoder");
-    SG_CUDA(cudaMemsetAsync(R.scalars.p, 0, 4 * 8, R.s));
+    SG_CUDA(cudaMemsetAsync(R.scalars.p, 0, 2 * 8, R.s));
 
     // Depth 0: the initial state is segment g0's layer; its children in the
     // other segments are collected at once (SetInitialNode,
     // DiskBasedOptThreeBitBFS.cpp:34-53).
     const uint64_t g0 = initial >> sb;
     {
-        SG_CUDA(cudaMemsetAsync(R.next.p, 0, R.seg_words * 8, R.s));
+        SG_CUDA(cudaMemsetAsync(R.next, 0, R.seg_words * 8, R.s));
+        SG_CUDA(cudaMemsetAsync(R.tally.p, 0, R.tally_bytes(), R.s));
         const uint64_t off = initial - g0 * R.seg_states;
         const uint64_t word = uint64_t(1) << (off & 63);
-        SG_CUDA(cudaMemcpyAsync(R.next.p + off / 64, &word, 8, cudaMemcpyHostToDevice, R.s));
-        if (int rc = R.found(R.next.p, g0, 1, *cur_s, *recv_s)) return rc;
+        SG_CUDA(cudaMemcpyAsync(R.next + off / 64, &word, 8, cudaMemcpyHostToDevice, R.s));
+        if (int rc = R.found(R.next, g0, 1, *cur_s, *recv_s)) return rc;
         cnt_cur[g0] = 1;
         if (int rc = R.stage_flush(*recv_s)) return rc;
     }
@@ -441,31 +440,31 @@ extern "C" int psb_bfs_segmented(const psb_puzzle* p, uint64_t initial, const ps
                 if (int rc = psb::store_erase(*old_s, int(g))) return rc;
                 continue;
             }
-            SG_CUDA(cudaMemsetAsync(R.next.p, 0, R.seg_words * 8, R.s));
-            if (int rc = R.receive(*recv_s, g, R.next.p)) return rc;
-            if (int rc = R.decode(*cur_s, R.cur.p, g, 0)) return rc;
+            SG_CUDA(cudaMemsetAsync(R.next, 0, 3 * R.seg_words * 8, R.s));
+            SG_CUDA(cudaMemsetAsync(R.tally.p, 0, R.tally_bytes(), R.s));
+            if (int rc = R.receive(*recv_s, g, R.next)) return rc;
+            if (int rc = R.decode(*cur_s, R.cur, g, 0)) return rc;
             if (cnt_cur[g])
-                if (int rc = R.expand_inside(R.cur.p, g)) return rc;
-            if (int rc = R.decode(*old_s, R.old.p, g, 1)) return rc;
-            SG_CUDA(cudaMemsetAsync(R.scalars.p, 0, 8, R.s));
-            psb::seg_finish<<<148 * 8, psb::kThreads, 0, R.s>>>(R.next.p, R.old.p, R.cur.p, R.seg_words, odd ? 1 : 0,
-                                                               R.scalars.p);
+                if (int rc = R.expand_inside(R.cur, g)) return rc;
+            if (int rc = R.decode(*old_s, R.old, g, 1)) return rc;
+            const unsigned fg = unsigned(std::min<uint64_t>((R.seg_words + psb::kThreads - 1) / psb::kThreads, 148 * 8));
+            psb::seg_finish<<<fg, psb::kThreads, 0, R.s>>>(R.next, R.old, R.cur, R.seg_words, odd ? 1 : 0, R.tally.p);
             SG_CUDA(cudaGetLastError());
-            SG_CUDA(cudaMemcpyAsync(R.pin, R.scalars.p, 8, cudaMemcpyDeviceToHost, R.s));
+            SG_CUDA(cudaMemcpyAsync(R.pin, R.tally.p, 8, cudaMemcpyDeviceToHost, R.s));
             SG_CUDA(cudaStreamSynchronize(R.s));
             const uint64_t c = R.pin[0];
             // g's depth d-1 layer is no longer needed (DeleteSegment of the old layer)
             if (int rc = psb::store_erase(*old_s, int(g))) return rc;
             total += c;
             cnt_new[g] = c;
-            if (int rc = R.found(R.next.p, g, c, *new_s, *next_s)) return rc;
+            if (int rc = R.found(R.next, g, c, *new_s, *next_s)) return rc;
             const uint64_t held = store_bytes();
             (R.files ? R.st.peak_disk_bytes : R.st.peak_host_bytes) =
                 std::max(R.files ? R.st.peak_disk_bytes : R.st.peak_host_bytes, held);
         }
         if (int rc = R.stage_flush(*next_s)) return rc;
         unsigned long long err[2] = {0, 0};
-        SG_CUDA(cudaMemcpyAsync(err, R.scalars.p + 2, 16, cudaMemcpyDeviceToHost, R.s));
+        SG_CUDA(cudaMemcpyAsync(err, R.scalars.p, 16, cudaMemcpyDeviceToHost, R.s));
         SG_CUDA(cudaStreamSynchronize(R.s));
         if (err[0]) return psb_set_error(PSB_ERR_DEVICE, "segmented search produced a child index >= IndexesCount()");
         if (err[1]) return psb_set_error(PSB_ERR_DEVICE, "segmented search: a layer decoded outside its segment");
@@ -485,7 +484,7 @@ extern "C" int psb_bfs_segmented(const psb_puzzle* p, uint64_t initial, const ps
     if (stats && stats->struct_size >= sizeof(psb_segmented_stats)) {
         R.st.struct_size = stats->struct_size;
         R.st.segments = S;
-        R.st.device_bytes = (R.next.cap + R.cur.cap + R.old.cap + R.kids.cap) * 8 + R.offs.cap * 4 +
+        R.st.device_bytes = (R.maps.cap + R.kids.cap) * 8 + R.offs.cap * 4 +
                             R.stream_buf[0].cap + R.stream_buf[1].cap;
         R.st.peak_host_bytes += R.stage.size() * 4;
         R.st.total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
