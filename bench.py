@@ -61,7 +61,7 @@ SPILL_BY_DEFAULT = {"pancake14-2bit", "hanoi18-2bit"}
 # inside the bench.  Used for roofline.traffic when the run has the same
 # launches (same level count, window and shape defaults).
 LEVEL_TRAFFIC = {
-    "pancake14-2bit": {"bytes": 11978881712384, "launches": 17, "window_bits": 16, "threads": 128,
+    "pancake14-2bit": {"bytes": 11441537860608, "launches": 17, "window_bits": 16, "threads": 128,
                        "profile": "profiles/level_kernel_pancake14_2bit_traffic.md"},
 }
 REF_SAMPLE = ("pancake", 11, 0, "two_bit")      # cpu_baseline: one reference InMemoryTwoBitBFS, one core
