@@ -1307,7 +1307,8 @@ int small_search(psb_bfs_session* S, uint64_t initial, uint32_t max_depth, int d
     a.ratio = ratio;
     a.pz = S->p.pz;
     // Two-bit runs the level of the last depth too (it counts the depth).
-    a.max_levels = !max_depth ? 0xFFFFFFFFu : S->algo == PSB_TWO_BIT ? max_depth + 1 : max_depth;
+    const uint64_t levels = uint64_t(max_depth) + (S->algo == PSB_TWO_BIT ? 1 : 0);
+    a.max_levels = max_depth ? uint32_t(std::min<uint64_t>(levels, 0xFFFFFFFFu)) : 0xFFFFFFFFu;
     a.bits = 10;
     while (S->p.n_states > uint64_t(psb::kSmallBlocks) << a.bits) a.bits++;
     a.direction = direction;
