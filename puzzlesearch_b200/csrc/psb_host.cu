@@ -886,6 +886,7 @@ constexpr uint64_t kSmallBottomUpStates = uint64_t(1) << 17;
 
 bool small_states(const psb_puzzle* p) {
     const bool hanoi = p->kind == PSB_HANOI4 || p->kind == PSB_HANOI4_OPT;
+    if (p->n_states > uint64_t(psb::kSmallBlocks) << psb::kSmallBitsMax) return false;
     if (hanoi && psb::hanoi_words_ok(p->pz)) return p->n_states <= kSmallHanoiStates;
     return p->n_states <= kSmallChildren / uint64_t(p->branching);
 }

@@ -1259,6 +1259,7 @@ __global__ void __launch_bounds__(kThreads) segment_expand_kernel(SegExpandArgs 
 // Whole searches of small puzzles in one launch (psb_small.cuh).
 // ---------------------------------------------------------------------------
 constexpr int kSmallBlocks = 16, kSmallThreads = 512;
+constexpr int kSmallBitsMax = 18;        // log2 of the most states a block holds (five bitmaps of them: 160 KB)
 constexpr uint32_t kSmallDepths = 1024;  // deeper searches run level by level
 constexpr int kSmallHeader = 7;          // words before the depths' (count, children) pairs
 constexpr int kSmallBottomUp = 2;        // SmallArgs::direction (PSB_DIR_BOTTOM_UP); 0: automatic

@@ -251,13 +251,21 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_search_kernel(SmallArg
     cluster.sync();  // no block leaves while others may still reach into it
 }
 
+// Dynamic shared memory of a block: its bitmaps and its warps' lists.
+__host__ __device__ constexpr size_t small_smem_bytes(size_t bitmaps, int bits) {
+    return bitmaps * (size_t(1) << bits) / 8 + kSmallThreads / 32 * 1024 * 2;
+}
+
+// The kernel's limit is the largest use, whatever this search takes: set to
+// each call's size, a smaller search on another thread could lower it between
+// this one's setting it and its launch.
 template <class PZ>
 cudaError_t launch_small_search(const SmallArgs& a, cudaStream_t s) {
-    const size_t bitmaps = a.mode == kThreeBit && a.arrays[0] ? 5 : 3;
-    const size_t smem = bitmaps * (size_t(1) << a.bits) / 8 + kSmallThreads / 32 * 1024 * 2;
+    const size_t smem = small_smem_bytes(a.mode == kThreeBit && a.arrays[0] ? 5 : 3, a.bits);
+    constexpr size_t limit = small_smem_bytes(5, kSmallBitsMax);
     cudaError_t e = cudaFuncSetAttribute(small_search_kernel<PZ>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(small_search_kernel<PZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        e = cudaFuncSetAttribute(small_search_kernel<PZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(limit));
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
