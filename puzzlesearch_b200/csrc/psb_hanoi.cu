@@ -43,8 +43,9 @@ cudaError_t launch_hanoi_level(const LevelArgs& a, unsigned grid, size_t smem, c
     if (!hanoi_words_ok(a.pz)) return launch_level<HanoiK, MODE, false, V>(a, grid, smem, s);
     constexpr int T = variant_threads(V);
     const size_t bytes = hanoi_smem_bytes(MODE, size_t(1) << a.window_bits, T);
+    constexpr size_t limit = hanoi_smem_bytes(MODE, size_t(1) << window_bits_max(MODE), T);  // as launch_level's
     cudaError_t e = cudaFuncSetAttribute(hanoi_level_kernel<MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(bytes));
+                                         int(limit));
     if (e != cudaSuccess) return e;
     // As many blocks as 148 SMs hold at once by threads; where shared memory
     // holds fewer, the rest queue up (no block waits for another).

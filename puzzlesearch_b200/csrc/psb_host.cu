@@ -1759,7 +1759,7 @@ int psb_bfs_session_create(const psb_puzzle* p, int algo, const psb_bfs_opts* op
     if (S->device < 0) PSB_CUDA(cudaGetDevice(&S->device));
     S->window_bits = (opts && opts->window_bits) ? opts->window_bits : auto_window_bits(p, algo);
     S->own_windows = !(opts && opts->window_bits);
-    if (S->window_bits < 10 || S->window_bits > 20 || (algo == PSB_FRONTIER && S->window_bits > 18))
+    if (S->window_bits < 10 || S->window_bits > psb::window_bits_max(S->mode))
         return fail(PSB_ERR_ARG, "window_bits %d out of range", S->window_bits);
     if (((p->n_states + (uint64_t(1) << S->window_bits) - 1) >> S->window_bits) > 0x7FFFFFFFull)
         return fail(PSB_ERR_ARG, "too many windows");

@@ -357,6 +357,9 @@ __host__ __device__ constexpr size_t level_smem_bytes(int mode, size_t window_st
            size_t(threads / 32) * (32 * states_per_unit(mode) * list_entry_bytes(mode) + kWarpScratch);
 }
 
+// The largest window a caller may ask for (psb_bfs_opts.window_bits).
+__host__ __device__ constexpr int window_bits_max(int mode) { return mode == kFrontier ? 18 : 20; }
+
 // Pancake operator 1 (flip of the last three values) only changes the two
 // lowest Lehmer digits: it maps index 6q + r to 6q + pi3(r) with
 // pi3 = (5 3 4 1 2 0), an involution, and n! is a multiple of 6.  So for a
@@ -1305,12 +1308,17 @@ cudaError_t launch_segment_expand(const SegExpandArgs& a, unsigned grid, cudaStr
     return cudaGetLastError();
 }
 
+// The kernel's shared-memory limit is the largest use, whatever this launch
+// takes: set to each launch's size, a search in smaller windows on another
+// thread could lower it between this one's setting it and its launch.
 template <class PZ, int MODE, bool BU = false, int V = 0>
 cudaError_t launch_level(const LevelArgs& a, unsigned grid, size_t smem, cudaStream_t s) {
+    constexpr int T = Shape<MODE, BU, V>::threads;
+    constexpr size_t limit = level_smem_bytes(MODE, size_t(1) << window_bits_max(MODE), T);
     cudaError_t e = cudaFuncSetAttribute(level_kernel<PZ, MODE, BU, V>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, int(limit));
     if (e != cudaSuccess) return e;
-    level_kernel<PZ, MODE, BU, V><<<grid, Shape<MODE, BU, V>::threads, smem, s>>>(a);
+    level_kernel<PZ, MODE, BU, V><<<grid, T, smem, s>>>(a);
     return cudaGetLastError();
 }
 

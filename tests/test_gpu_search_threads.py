@@ -40,3 +40,21 @@ def test_one_launch_searches():
 
     assert not together(search(11, 2000), search(11, 2000), search(9, 2000), search(9, 2000))
     assert set(whole[9]) == set(whole[11]) == {1}
+
+@pytest.mark.parametrize("algo", ["two_bit", "three_bit", "frontier"])
+@pytest.mark.parametrize("puzzle", ["hanoi", "sliding"])
+def test_level_kernels(puzzle, algo):
+    """Windows of different size in the two threads: 64 KB and more of marks against 1 KB."""
+    wide = 18 if algo == "frontier" else 20
+    p = psb.FourPegHanoiSimple(7) if puzzle == "hanoi" else psb.SlidingTilePuzzleSimple(3, 3)
+    want = psb.bfs(p, algo, 0)["counts"]
+    got = []
+
+    def search(window_bits):
+        def job():
+            for _ in range(60):
+                got.append(psb.bfs(p, algo, 0, window_bits=window_bits, threads=256)["counts"])
+        return job
+
+    assert not together(search(wide), search(10), search(10))
+    assert len(got) == 180 and all(c == want for c in got)
