@@ -19,6 +19,7 @@
 #include "psb_hanoi_words.cuh"
 #include "psb_internal.h"
 #include "psb_kernels.cuh"
+#include "psb_launch.h"
 
 using psb::LevelArgs;
 using psb::PuzzleArgs;
@@ -1294,8 +1295,9 @@ int spill_depth(psb_bfs_session* S, const psb_bfs_opts* o, uint32_t depth, const
 }
 
 // Runs a whole search in one launch (psb_small.cuh): S->h_stats holds
-// its result afterwards.  *done false: too deep for it, or no cluster of that
-// size here; nothing has happened to the session that a search does not reset.
+// its result afterwards.  *done false: too deep for it, or the device has no
+// room for the cluster; nothing has happened to the session that a search does
+// not reset.
 int small_search(psb_bfs_session* S, uint64_t initial, uint32_t max_depth, int direction, double ratio, bool can_bu,
                  bool arrays, bool* done) {
     psb::SmallArgs a{};
@@ -1315,10 +1317,12 @@ int small_search(psb_bfs_session* S, uint64_t initial, uint32_t max_depth, int d
     a.direction = direction;
     a.can_bu = can_bu ? 1 : 0;
     *done = false;
-    if (S->p.k.small(a, S->stream) != cudaSuccess) {
+    const cudaError_t launched = S->p.k.small(a, S->stream);
+    if (psb::launch_has_no_room(launched)) {
         cudaGetLastError();
         return PSB_OK;
     }
+    PSB_CUDA(launched);
     PSB_CUDA(cudaMemcpyAsync(S->h_stats, a.out, kSmallOut * 8, cudaMemcpyDeviceToHost, S->stream));
     PSB_CUDA(cudaStreamSynchronize(S->stream));
     if (S->h_stats[0] == 1) return fail(PSB_ERR_DEVICE, "level kernel produced a child index >= IndexesCount()");
