@@ -741,8 +741,8 @@ def frontier_encode(d_bits, first_bit, n_bits, d_out=None, out_cap=0, stream=Non
     (stream_bytes, block_table, n_blocks); with d_out=None only sizes it."""
     nbytes = ctypes.c_uint64()
     nb = ctypes.c_uint32()
-    # as many blocks as the range can hold (262,144 offsets each)
-    rows = 0 if d_out is None else max(1, (n_bits + 262143) // 262144)
+    # as many blocks as the range can hold (262,144 offsets each); the library refuses ranges past 2^32
+    rows = 0 if d_out is None else max(1, (min(n_bits, 1 << 32) + 262143) // 262144)
     blocks = (CodecBlock * rows)() if rows else None
     rc = lib().psb_frontier_encode(ctypes.cast(d_bits, u64p), first_bit, n_bits, d_out, out_cap,
                                    ctypes.byref(nbytes), blocks, rows, ctypes.byref(nb), stream)
