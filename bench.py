@@ -59,11 +59,27 @@ SPILL_BY_DEFAULT = {"pancake14-2bit", "hanoi18-2bit"}
 # kernels over one full search, from a one-pass ncu capture of the same search
 # without spill (the level launches are the same with it); ncu cannot run
 # inside the bench.  Used for roofline.traffic when the run has the same
-# launches (same level count, window and shape defaults).
+# launches (recorded_traffic).
 LEVEL_TRAFFIC = {
     "pancake14-2bit": {"bytes": 11441537860608, "launches": 17, "window_bits": 16, "threads": 128,
                        "profile": "profiles/level_kernel_pancake14_2bit_traffic.md"},
 }
+
+
+def recorded_traffic(args, st):
+    """The capture whose launches are this run's, or None: the same level
+    count, window and block size, the window not asked for (one that is asked
+    for runs another kernel and reports the same size), far marks NEAR (the
+    automatic choice), direction and bottom-up ratio automatic."""
+    tr = LEVEL_TRAFFIC.get(args.workload)
+    if not tr or args.window_bits or args.far_marks not in ("auto", "near"):
+        return None
+    if args.direction != "auto" or args.bottom_up_ratio:
+        return None
+    same = (st.levels, st.window_bits, st.threads) == (tr["launches"], tr["window_bits"], tr["threads"])
+    return tr if same else None
+
+
 REF_SAMPLE = ("pancake", 11, 0, "two_bit")      # cpu_baseline: one reference InMemoryTwoBitBFS, one core
 REF_ARM_SAMPLE = ("pancake", 10, 0, "two_bit")  # --impl reference: one search per host core per step
 
@@ -616,8 +632,8 @@ def main():
     achieved = alg_bytes / (expand_ms / 1000.0) / 1e9
     peak, peak_kind = load_peaks()
     traffic = None
-    tr = LEVEL_TRAFFIC.get(args.workload)
-    if tr and st.levels == tr["launches"] and st.window_bits == tr["window_bits"] and st.threads == tr["threads"]:
+    tr = recorded_traffic(args, st)
+    if tr:
         traffic = {"per_launch": tr["bytes"] / tr["launches"], "per_search": tr["bytes"],
                    "vs_algorithmic": tr["bytes"] / alg_bytes,
                    # the captured bytes over this run's level time: the DRAM throughput the kernels sustain
