@@ -80,6 +80,7 @@ def recorded_traffic(args, st):
     return tr if same else None
 
 
+ENGINE_BLOCKS_PER_SM = 4  # psb_engine_opts.blocks_per_sm = 0
 REF_SAMPLE = ("pancake", 11, 0, "two_bit")      # cpu_baseline: one reference InMemoryTwoBitBFS, one core
 REF_ARM_SAMPLE = ("pancake", 10, 0, "two_bit")  # --impl reference: one search per host core per step
 
@@ -347,7 +348,7 @@ def batch_bench(args):
             "higher_is_better": True, "dtype": "u64", "data": "seeded random solvable starts",
             "config": {"workload": "batch4096", "instances": len(items), "states": total_states,
                        "engine_levels": levels, "direction": direction,
-                       "blocks_per_sm": blocks_per_sm or 2, "window_bits_offset": wb_offset,
+                       "blocks_per_sm": blocks_per_sm or ENGINE_BLOCKS_PER_SM, "window_bits_offset": wb_offset,
                        "autotune": tuning},
             "batched": {"seconds": b_dt, "solves_per_s": len(items) / b_dt, "states_per_s": total_states / b_dt},
             "plain_one_per_launch": {"seconds": p_dt, "solves_per_s": len(items) / p_dt,

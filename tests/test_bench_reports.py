@@ -1,5 +1,7 @@
 """What bench.py reports beside its times: the recorded DRAM traffic belongs to
-the launches of the run."""
+the launches of the run, and the engine's default grid is the library's."""
+import os
+import re
 from types import SimpleNamespace
 
 import pytest
@@ -28,3 +30,11 @@ def test_traffic_of_the_captured_launches():
 def test_no_traffic_of_other_launches(change):
     """A window that is asked for reports the size of the automatic one and runs another kernel."""
     assert run(**change) is None
+
+
+def test_default_engine_grid():
+    header = open(os.path.join(bench.REPO, "include", "psb200.h")).read()
+    engine = open(os.path.join(bench.REPO, "puzzlesearch_b200", "csrc", "psb_engine.cu")).read()
+    blocks = int(re.search(r"kEMinBlocks = (\d+);", engine).group(1))
+    assert f"persistent blocks per SM (0 = {blocks})" in header
+    assert bench.ENGINE_BLOCKS_PER_SM == blocks
