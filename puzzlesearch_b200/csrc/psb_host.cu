@@ -1465,6 +1465,12 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
         }
         if (S->algo != PSB_TWO_BIT && h[6]) res.push_back(h[6]);  // the depth that the last level found
     }
+    auto with_flags = [&](SpillSource& src) {  // those of the depth that the next level would expand
+        if (flags_valid < 0) return;
+        src.flags = S->wflags[flags_valid];
+        src.window_bits = S->window_bits;
+        src.n_windows = S->n_windows;
+    };
     while (!whole) {
         if (max_depth && res.size() >= size_t(max_depth) + 1) break;
         if (spill) {  // the states at depth `iteration`, before its level changes the arrays
@@ -1479,11 +1485,7 @@ int session_run(psb_bfs_session* S, uint64_t initial, const psb_bfs_opts* opts, 
                 src.ops = true;
                 break;
             }
-            if (flags_valid >= 0) {
-                src.flags = S->wflags[flags_valid];
-                src.window_bits = S->window_bits;
-                src.n_windows = S->n_windows;
-            }
+            with_flags(src);
             if (int rc = spill_depth(S, opts, iteration, src, &spilled)) return rc;
             spilled_depths = iteration + 1;
         }
@@ -1677,6 +1679,7 @@ done:
         // last depth, which no level expanded, in cur / open.
         SpillSource src;
         src.bitmap = S->algo == PSB_THREE_BIT ? cur : open;
+        with_flags(src);
         if (int rc = spill_depth(S, opts, spilled_depths, src, &spilled)) return rc;
     }
     if (spill) if (int rc = spill_drain(S->spill, opts, &spilled)) return rc;
