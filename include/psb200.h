@@ -255,10 +255,12 @@ int psb_bfs_session_destroy(psb_bfs_session* s);
 
 /* Search arrays (psb_bfs and sessions) come from a per-device memory pool
  * that keeps freed memory reserved for the next search instead of returning
- * it to the driver after every call.  This returns the reserved memory of
+ * it to the driver after every call; the scratch of psb_frontier_encode and
+ * psb_frontier_decode comes from it too.  This returns the reserved memory of
  * `device` (-1 = current) to the driver, and frees the frontier spill's
- * cached buffers and the streams, events and pinned words kept for the next
- * searches (at most 8 sets a device); it waits for the device first. */
+ * cached buffers, the streams, events and pinned words kept for the next
+ * searches (at most 8 sets a device) and the pinned blocks kept for the next
+ * segmented searches (at most 4 of 1.1 MB); it waits for the device first. */
 int psb_release_cached_memory(int device);
 
 /* --- Device bit arrays (Common/BitArray.h:69-169) -------------------------

@@ -1846,6 +1846,7 @@ int psb_release_cached_memory(int device) {
         sessions.swap(g_session_cache[device]);
     }
     for (SessionRes* R : sessions) delete R;
+    psb::segmented_release();
     if (!pool) return PSB_OK;
     PSB_CUDA(cudaDeviceSynchronize());  // frees still queued on streams return first
     PSB_CUDA(cudaMemPoolTrimTo(pool, 0));

@@ -92,6 +92,9 @@ int store_read(StoreImpl& s, int segment, void* buf, uint64_t cap, uint64_t* got
 int store_erase(StoreImpl& s, int segment);
 int store_erase_all(StoreImpl& s);
 
+// Frees the pinned host blocks that segmented searches keep (psb_segmented.cu).
+void segmented_release();
+
 // The current device's memory pool (psb_release_cached_memory trims it).
 int scratch_pool(cudaMemPool_t* pool);
 // Decodes a segment stream (block table on the host) into the bitmap

@@ -28,6 +28,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -110,6 +111,37 @@ struct DevBuf {
     }
 };
 
+// Pinned host blocks of kPinBlock bytes kept for the next calls, at most
+// kPinKept of them.  A call's own block took 0.2 ms to make and up to 2 ms to
+// free (freeing waits for the device), more than a small search.
+constexpr uint64_t kPinBlock = 2 * kPinned + (uint64_t(1) << 17);  // enough for 2^14 segments
+constexpr size_t kPinKept = 4;
+std::mutex g_pin_mu;
+std::vector<void*> g_pin_kept;
+
+cudaError_t pin_acquire(uint64_t bytes, void** out) {
+    if (bytes <= kPinBlock) {
+        std::lock_guard<std::mutex> lock(g_pin_mu);
+        if (!g_pin_kept.empty()) {
+            *out = g_pin_kept.back();
+            g_pin_kept.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaMallocHost(out, std::max(bytes, kPinBlock));
+}
+
+void pin_return(void* p, uint64_t bytes) {  // no copy to or from it is in flight
+    if (bytes <= kPinBlock) {
+        std::lock_guard<std::mutex> lock(g_pin_mu);
+        if (g_pin_kept.size() < kPinKept) {
+            g_pin_kept.push_back(p);
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
 struct Run {
     const psb_puzzle* P = nullptr;
     cudaStream_t s = nullptr;
@@ -144,13 +176,14 @@ struct Run {
         if (enc) psb::encoder_destroy(enc);
         if (dec) psb::decoder_destroy(dec);  // frees its scratch in stream order
         if (s) cudaStreamDestroy(s);
-        if (pin) cudaFreeHost(pin);
+        if (pin) pin_return(pin, pin_bytes());
     }
 
+    uint64_t pin_bytes() const { return (tally_bytes() + 15) / 16 * 16 + (n_segments + 3) / 4 * 16 + 2 * kPinned; }
     int pin_host() {
         const uint64_t tally = (tally_bytes() + 15) / 16 * 16, runs = (n_segments + 3) / 4 * 16;
         void* v = nullptr;
-        SG_CUDA(cudaMallocHost(&v, tally + runs + 2 * kPinned));
+        SG_CUDA(pin_acquire(pin_bytes(), &v));
         pin = static_cast<unsigned long long*>(v);
         pin_hist = reinterpret_cast<unsigned int*>(pin + 2);
         pin_start = reinterpret_cast<unsigned int*>(static_cast<uint8_t*>(v) + tally);
@@ -340,6 +373,15 @@ struct Run {
 };
 
 }  // namespace
+
+void psb::segmented_release() {
+    std::vector<void*> kept;
+    {
+        std::lock_guard<std::mutex> lock(g_pin_mu);
+        kept.swap(g_pin_kept);
+    }
+    for (void* p : kept) cudaFreeHost(p);
+}
 
 extern "C" int psb_bfs_segmented(const psb_puzzle* p, uint64_t initial, const psb_segmented_opts* opts,
                                  uint64_t* counts, uint32_t cap, uint32_t* n_depths, psb_segmented_stats* stats) {
