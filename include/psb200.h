@@ -146,7 +146,11 @@ enum { PSB_FAR_AUTO = 0, PSB_FAR_NONE = 1, PSB_FAR_NEAR = 2, PSB_FAR_ALL = 3 };
 typedef struct {
     uint32_t struct_size;  /* sizeof(psb_bfs_opts) */
     uint32_t max_depth;    /* stop after this depth (0 = until the frontier is empty; PuzzleOptions::maxSteps, Common/DiskBasedBFS.h:10) */
-    int32_t window_bits;   /* log2 states per thread-block window (0 = automatic) */
+    int32_t window_bits;   /* log2 states per thread-block window (0 = automatic).  A size that is asked for, the one
+                              that psb_bfs_stats reports too, runs the kernels of windows of 2^window_bits states level
+                              by level; only 0 lets pancakes of 11 and more take windows of 8! states and small
+                              searches run in one launch, which far_marks, threads, level_ms, spill and
+                              restored_counts also turn off */
     int32_t device;        /* CUDA device ordinal (-1 = current) */
     void* stream;          /* cudaStream_t (NULL = a stream owned by the call) */
     uint64_t* final_words; /* optional host buffer: final arrays in the reference's layout (see psb_final_words) */
@@ -204,7 +208,7 @@ typedef struct {
 typedef struct {
     uint32_t struct_size;     /* sizeof(psb_bfs_stats) */
     uint32_t levels;          /* BFS levels run */
-    uint32_t window_bits;     /* window used */
+    uint32_t window_bits;     /* window used (with windows of 8! states: the states per active-window flag) */
     uint32_t threads;         /* threads per block of the level kernel */
     double total_ms;          /* device time of the whole search (CUDA events) */
     double expand_ms;         /* sum over levels of the fused sweep+expand+mark kernel */

@@ -20,8 +20,8 @@
 // takes about 250 here whatever number of its states is in the frontier.
 // Units holding frontier states are queued per warp and expanded 32 at a
 // time, so sparse chunks do not leave lanes idle.  17 disks, two-bit, whole
-// search on B200: 444 -> 105 ms; a dense level of 15 disks 757 -> 191 us, the
-// ALU pipe at 52%, DRAM at 19%, a quarter of the stalls at window barriers.
+// search on B200: 444 -> 102 ms; a dense level of 15 disks 757 -> 197 us, the
+// ALU pipe at 53%, DRAM at 19%, an eighth of the stalls at window barriers.
 //
 // Marks of a unit are one 64-bit mask in shared memory (four for frontier
 // search, one per operator) in the unit's bit order, which is the order its

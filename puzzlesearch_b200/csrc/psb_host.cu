@@ -1049,7 +1049,8 @@ int layout(const psb_puzzle* p, int algo, uint64_t* words, int* n_arr) {
 // puzzle, and it fails for Hanoi with symmetry, whose index space also holds
 // non-canonical states that expand to canonical children.  Frontier search
 // keeps no visited information.
-// Default switch ratio of PSB_DIR_AUTO (unvisited < ratio x frontier).
+// Default switch ratio of PSB_DIR_AUTO (unvisited < ratio x frontier), swept
+// with the bottom-up kernel that computed factorials at run time, twice as slow.
 constexpr double kBottomUpRatio = 1.0;
 
 // PSB_FAR_AUTO's pick (measured on B200, two-bit, full searches):
@@ -1092,8 +1093,9 @@ size_t smem_bytes(int mode, int wb, int threads = 0) {
 // threads = 0, two-bit pancake and Hanoi searches of 2^32 states or more take
 // 128-thread blocks, five per SM (B200, whole search, far marks NEAR, windows
 // of 2^16: 14-pancake 4.06 s at 128 threads vs 4.40 s at 256).  In windows of
-// 8! states the two are within 2% (14-pancake 2.93 vs 2.86 s, 13-pancake 138
-// vs 135 ms).  Two-bit Hanoi without symmetry (64 states at a time,
+// 8! states 256 is 2% faster (14-pancake 2.93 vs 2.86 s, 13-pancake 138 vs
+// 135 ms); 128 stays the number that such a search reports
+// (tests/test_gpu_large.py holds it).  Two-bit Hanoi without symmetry (64 states at a time,
 // psb_hanoi_words.cuh) takes them at any size: a window's warps finish closer
 // together (18 disks 358 vs 393 ms).  Three-bit (13-pancake 157 vs 152 ms) and
 // the sliding-tile puzzles (3x4 two-bit 10.5 vs 10.7 ms) keep 256.

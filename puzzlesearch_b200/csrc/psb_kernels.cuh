@@ -57,7 +57,8 @@ enum Mode : int { kThreeBit = 0, kClassic = 1, kTwoBit = 2, kFrontier = 3 };
 // 13-pancake 213 ms against 226 ms with four blocks of 128 registers,
 // 14-pancake 4.06 s against 4.15 s).  The 13- and 14-pancake kernels issue their far reads
 // early and keep them in flight across the near children, which needs
-// registers rather than warps (at 64 registers they spill).
+// registers rather than warps (79 and 84 used at 128 threads; at 64 the
+// 14-pancake one spills).
 template <int MODE, bool BU = false, int V = 0>
 struct Shape {
     static constexpr int threads = V == 1 ? 512 : V == 2 ? 128 : 256;
@@ -89,7 +90,7 @@ struct PuzzleArgs {
 // kPairOp0: operator 0 maps state i to i ^ 1 (the pancake flip of the last
 // two values only toggles the lowest Lehmer digit, of weight 1!), so a level
 // kernel can mark those children for a whole frontier word at once and expand
-// the rest with expand_from<1>.
+// the rest with expand_from_prefixed<1>.
 // kChunkPrefix: the level kernel unranks the shared leading positions of a
 // chunk's states once (make_prefix, two blocks of 7! indexes at most per
 // chunk) and each state's remaining positions from index % 7!.
